@@ -14,10 +14,11 @@
 //                        (BatchDecodeWithPagedKVCacheKernel, decode.cuh:451-620)
 //
 // Decode is HBM-bound: every K and V entry of a (request, kv head) is read exactly once, whatever the
-// number of query heads that share the kv head - they are the rows of one tensor-core tile.  Long
-// sequences of small batches are cut into `splits` ranges of key tiles so that the machine is filled; the
+// number of query heads that share the kv head - they are the columns of one tensor-core tile.  Long
+// sequences of small batches are cut into up to `splits` ranges of key tiles so that the machine is filled; the
 // partial softmax states go through a workspace and the CTA that finishes last (a ticket, no waiting)
-// merges them in range order - a fixed order, so the result does not depend on scheduling.
+// merges them in range order - a fixed order, so the result does not depend on scheduling.  In batches that
+// need no ranges the longest requests go first, so that the launch ends on its shortest CTAs.
 #pragma once
 #include "smlm_common.cuh"
 
@@ -38,6 +39,8 @@ struct PdArgs {
   int* tickets;                   // [B * Nkv], zero between launches
   float* partial;                 // [B * Nq * splits * kPdRec]
   int batch, num_kv_heads, num_layers, layer_idx, page_size, splits, total_pages;
+  int min_tiles;                  // a range is not made shorter than this many tiles
+  int sorted;                     // 1: CTAs take the requests in descending order of their length (batch <= kPdMaxSorted)
   float log2_theta;               // log2(rope base)
 };
 
@@ -127,39 +130,50 @@ __global__ void __launch_bounds__(128) append_kv_kernel(const AppendArgs a) {
 // decode
 // ---------------------------------------------------------------------------------------------
 
-// online-softmax state merge in the base-2 domain for N values: (m, d, o) <- (m, d, o) + (m2, d2, o2)
-template <int N>
-__device__ __forceinline__ void pd_merge(float& m, float& d, float (&o)[N], float m2, float d2, const float (&o2)[N]) {
-  if (d2 == 0.f) return;             // an empty state carries no information (and its m may be -inf)
-  if (d == 0.f) {
-    m = m2; d = d2;
-#pragma unroll
-    for (int i = 0; i < N; ++i) o[i] = o2[i];
-    return;
-  }
-  const float mn = fmaxf(m, m2);
-  const float s1 = exp2f(m - mn), s2 = exp2f(m2 - mn);
-  d = d * s1 + d2 * s2;
-#pragma unroll
-  for (int i = 0; i < N; ++i) o[i] = o[i] * s1 + o2[i] * s2;
-  m = mn;
-}
-
 constexpr int kPdWarps = 4;                          // each warp streams its own tiles of 16 keys
 constexpr int kPdTile = 16;
 constexpr int kPdTileBytes = kPdTile * kPdDim * 2;   // one tile of K (or V) of one head: 4 KB
 constexpr int kPdWarpRing = kPdStages * 2 * kPdTileBytes;
-constexpr int kPdQOff = kPdWarps * kPdWarpRing;      // rotated queries [8 rows][128], then 16 bytes of zeros
-constexpr int kPdSmem = kPdQOff + 8 * kPdDim * 2 + 64;
+constexpr int kPdQOff = kPdWarps * kPdWarpRing;      // rotated queries [8 rows][128]
+constexpr int kPdRotOff = kPdQOff + 8 * kPdDim * 2;  // frequency pairs: step of a warp, step of 8 keys, frequencies
+constexpr int kPdSmem = kPdRotOff + 2 * 512 + 256;
+constexpr int kPdStep = kPdWarps * kPdTile;          // keys between two tiles of a warp
+constexpr int kPdMaxSorted = 512;                    // requests whose ranks a CTA finds for itself
+constexpr int kPdReseed = 16;                        // tiles after which the rotation is computed afresh
+constexpr float kPdRaise = 8.0f;                     // a head's maximum is raised when exceeded by this much (log2)
 
-// One CTA = one (request, kv head, range of key tiles).  The G query heads that share the kv head are the
-// rows of a 16-row MMA tile (rows G..15 are zero), so every key and value is read once for all of them:
-//   S[heads, 16 keys] = Q . K^T  and  O[heads, 128] += P . V  with mma.sync m16n8k16, fp32 accumulation.
+// 8 x 8 transpose of 16-bit elements over a warp
+__device__ __forceinline__ uint32_t movm_t(uint32_t v) {
+  uint32_t r;
+  asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;\n" : "=r"(r) : "r"(v));
+  return r;
+}
+// (c, s) of an angle turned by (c1, s1), two angles at once
+__device__ __forceinline__ void turn_f32x2(uint64_t& c, uint64_t& s, uint64_t c1, uint64_t s1) {
+  const uint64_t n = fma_f32x2(c, c1, mul_f32x2(s ^ 0x8000000080000000ull, s1));
+  s = fma_f32x2(s, c1, mul_f32x2(c, s1));
+  c = n;
+}
+
+// One CTA = one (request, kv head, range of key tiles).  The keys of a tile are the rows of the MMA and the
+// G query heads that share the kv head its columns, so every key and value is read once for all of them and no
+// row is padding:
+//   S^T[16 keys, 8 heads] = K . Q^T  and  O^T[128, 8 heads] += V^T . P^T  with mma.sync m16n8k16, fp32 accumulation.
 // Each warp owns every fourth tile of the range and a private ring of shared-memory stages filled with
-// 16-byte cp.async copies (no CTA-wide barrier in the loop).  A tile's keys are rotated where they lie in
-// shared memory before the MMA reads them: lane l owns the frequency pair (2l, 2l+1) and walks the 16
-// positions of the tile with the angle-addition recurrence, re-seeded exactly at every tile.  The rotated
-// keys are rounded to the storage type - what a cache that stores rotated keys holds anyway.
+// 16-byte cp.async copies (no CTA-wide barrier in the loop).
+//
+// The keys are rotated in registers between ldmatrix and the MMA: a lane's fragments hold, for keys g and g + 8
+// of the tile, a dimension and (four k steps later) its partner 64 dimensions on.  A lane keeps the cosines and
+// sines of key g for its 16 frequencies, turns them by 8 keys for the other key and by the warp's step for its next
+// tile, and computes them afresh every 16 tiles (16 turns: the error of one).  The rotated keys are rounded to
+// the storage type - what a cache that stores rotated keys holds anyway.
+//
+// What bounds it: with the keys' rows rotated in place in shared memory (two loads and two stores per key and
+// lane) and the heads as the rows of a half-empty tile, a tile of 16 keys took a warp about 960 instructions and
+// the 12 warps of an SM could not issue them as fast as the keys arrive; this form needs under half.  A head's
+// maximum is only raised when it is exceeded by more than 2^8 (one vote per tile instead of six shuffles).
+// Measured, append + decode of 128 requests with contexts 512..4096, 32 / 8 heads (1236 MB): 287 us before, 215 us
+// now (5.75 TB/s), with the longest requests first.
 template <typename T, int G>
 __global__ void __launch_bounds__(kPdWarps * 32, 3) paged_decode_kernel(const PdArgs a) {
   extern __shared__ __align__(128) unsigned char pd_smem[];
@@ -167,18 +181,39 @@ __global__ void __launch_bounds__(kPdWarps * 32, 3) paged_decode_kernel(const Pd
   const int tid = threadIdx.x;
   const int lane = tid & 31;
   const int warp = tid >> 5;
-  const int g = lane >> 2, t = lane & 3;       // MMA fragment coordinates: row (head) g, column pair t
+  const int g = lane >> 2, t = lane & 3;       // MMA fragment coordinates: row g, column pair t
 
   const int S = a.splits;
   const int s = blockIdx.x % S;
-  const int bh = blockIdx.x / S;
-  const int kvh = bh % a.num_kv_heads;
-  const int b = bh / a.num_kv_heads;
+  const int kvh = blockIdx.x / S % a.num_kv_heads;
+  int b = blockIdx.x / S / a.num_kv_heads;
   const int Nq = a.num_kv_heads * G;
   const int P = a.page_size;
   const int head0 = kvh * G;
 
   pdl_wait();
+  if (a.sorted) {
+    // the request whose number of pages has rank b: every CTA counts for itself (whatever the table holds, the
+    // ranks are a permutation of the requests)
+    int* len = reinterpret_cast<int*>(pd_smem);
+    const int n4 = (a.batch + 3) & ~3;
+    for (int i = tid; i < n4; i += kPdWarps * 32) len[i] = i < a.batch ? a.kv_indptr[i + 1] - a.kv_indptr[i] : INT32_MIN;
+    __syncthreads();
+    for (int i = tid; i < a.batch; i += kPdWarps * 32) {
+      const int mine = len[i];
+      int rank = 0;
+      for (int k = 0; k < n4; k += 4) {   // (entries past the batch are never ahead: smallest, and behind)
+        const int4 v = *reinterpret_cast<const int4*>(len + k);
+        rank += (v.x > mine || (v.x == mine && k < i)) + (v.y > mine || (v.y == mine && k + 1 < i)) +
+                (v.z > mine || (v.z == mine && k + 2 < i)) + (v.w > mine || (v.w == mine && k + 3 < i));
+      }
+      if (rank == b) s_last = i;
+    }
+    __syncthreads();
+    b = s_last;
+    __syncthreads();   // the ranks' space is the ring's, s_last serves the ranges later
+  }
+  const int bh = b * a.num_kv_heads + kvh;
   int p0 = a.kv_indptr[b], p1 = a.kv_indptr[b + 1];
   if (p0 < 0 || p1 < p0 || p1 > a.total_pages) {
     if (tid == 0 && a.err != nullptr) atomicOr(a.err, kErrBadIndptr);
@@ -192,7 +227,9 @@ __global__ void __launch_bounds__(kPdWarps * 32, 3) paged_decode_kernel(const Pd
   }
   const int seq_len = npages > 0 ? (npages - 1) * P + last_valid : 0;
   const int ntiles = (seq_len + kPdTile - 1) / kPdTile;
-  const int per = (ntiles + S - 1) / S;
+  const int per = max((ntiles + S - 1) / S, a.min_tiles);
+  const int ranges = max(1, (ntiles + per - 1) / per);        // ranges this request is cut into
+  if (s >= ranges) return;
   const int tile0 = s * per;
   const int ntl = max(0, min(ntiles, tile0 + per) - tile0);   // tiles of this CTA
   const int ntw = ntl > warp ? (ntl - warp + kPdWarps - 1) / kPdWarps : 0;   // tiles of this warp
@@ -230,17 +267,32 @@ __global__ void __launch_bounds__(kPdWarps * 32, 3) paged_decode_kernel(const Pd
                  "r"(pack2<T>(ro[0], ro[1])), "r"(pack2<T>(ro[2], ro[3])) : "memory");
     asm volatile("st.shared.v2.b32 [%0], {%1, %2};\n" ::"r"(qs + row * 256 + ((c_par ^ row) << 4) + off),
                  "r"(pack2<T>(rp[0], rp[1])), "r"(pack2<T>(rp[2], rp[3])) : "memory");
-    if (tid < 4) asm volatile("st.shared.b32 [%0], %1;\n" ::"r"(qs + 8 * 256 + tid * 4), "r"(0) : "memory");
+  }
+  // the turns by the warp's step and by 8 keys, and the frequencies: (cos, cos, sin, sin) of two frequencies each
+  float* rot = reinterpret_cast<float*>(pd_smem + kPdRotOff);
+  if (tid < 64) {
+    const float f = exp2f(-a.log2_theta * static_cast<float>(2 * tid) * (1.0f / kPdDim)) * 0.31830988618379067f;
+    float sn, cs;
+    float* r = rot + (tid >> 1) * 4 + (tid & 1);
+    sincospif(static_cast<float>(kPdStep) * f, &sn, &cs);
+    r[0] = cs;
+    r[2] = sn;
+    sincospif(8.0f * f, &sn, &cs);
+    r[128] = cs;
+    r[130] = sn;
+    rot[256 + tid] = f;
   }
   __syncthreads();
-  uint32_t qf[8][4];
+  uint32_t qf[8][2];   // B operand: dimensions 16 ks ..., column = head
 #pragma unroll
-  for (int ks = 0; ks < 8; ++ks) {
-    // matrices: (rows 0-7, k lo), (rows 8-15, k lo), (rows 0-7, k hi), (rows 8-15, k hi); rows 8-15 are zeros
-    const int m = lane >> 3, r = lane & 7;
-    const int chunk = ks * 2 + (m >> 1);
-    const uint32_t addr = (m & 1) ? qs + 8 * 256 : qs + r * 256 + ((chunk ^ r) << 4);
-    ldsm_x4(qf[ks], addr);
+  for (int i = 0; i < 4; ++i) {
+    const int r = lane & 7, chunk = 4 * i + (lane >> 3);
+    uint32_t f4[4];
+    ldsm_x4(f4, qs + r * 256 + ((chunk ^ r) << 4));
+    qf[2 * i][0] = f4[0];
+    qf[2 * i][1] = f4[1];
+    qf[2 * i + 1][0] = f4[2];
+    qf[2 * i + 1][1] = f4[3];
   }
 
   // ---- this warp's ring and its loader ----
@@ -268,20 +320,27 @@ __global__ void __launch_bounds__(kPdWarps * 32, 3) paged_decode_kernel(const Pd
       }
     }
   };
+  // lane l copies chunk l & 15 of the keys 2 k + (l >> 4); chunk c of key e sits at slot c ^ (e & 7)
+  const int cch = lane & 15, ckey = lane >> 4;
+  const uint32_t dst_row = ckey * 256;
   auto issue = [&](int j) {   // j-th tile of this warp; its addresses were looked up before
     if (j < ntw) {
       const int key0 = (tile0 + warp + j * kPdWarps) * kPdTile;
-      const uint32_t kst = ring + (j % kPdStages) * (2 * kPdTileBytes);
-      const int cch = lane & 15;
+      const uint32_t kst = ring + (j % kPdStages) * (2 * kPdTileBytes) + dst_row;
+      const int valid = seq_len - key0 - ckey;   // key 2 k of this lane exists if 2 k < valid
 #pragma unroll
-      for (int k = 0; k < kPdTile / 2; ++k) {
-        const int key = 2 * k + (lane >> 4);
-        const T* hp = half_ptr[k >> 2];
-        const bool ok = hp != nullptr && key0 + key < seq_len;
-        const T* src = ok ? hp + (key & 7) * kPdDim + cch * 8 : static_cast<const T*>(a.q);
-        const uint32_t dst = kst + key * 256 + ((cch ^ (key & 7)) << 4);
-        cp_async16(dst, src, ok);                                             // keys past the end read as zeros
-        cp_async16(dst + kPdTileBytes, ok ? src + kv_delta : src, ok);
+      for (int h = 0; h < 2; ++h) {
+        const bool have = half_ptr[h] != nullptr;
+        const T* src = have ? half_ptr[h] + ckey * kPdDim + cch * 8 : static_cast<const T*>(a.q);
+        const T* vsrc = have ? src + kv_delta : src;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const bool ok = have && 8 * h + 2 * k < valid;                    // keys past the end read as zeros
+          const int step = ok ? 2 * k * kPdDim : 0;
+          const uint32_t dst = kst + (8 * h + 2 * k) * 256 + ((cch ^ (2 * k + ckey)) << 4);
+          cp_async16(dst, src + step, ok);
+          cp_async16(dst + kPdTileBytes, vsrc + step, ok);
+        }
       }
     }
     cp_async_commit();
@@ -291,198 +350,206 @@ __global__ void __launch_bounds__(kPdWarps * 32, 3) paged_decode_kernel(const Pd
 #pragma unroll
   for (int j = 0; j < kPdStages - 1; ++j) issue(j);
 
-  // ---- rotation state of this lane: frequencies 2l and 2l + 1 ----
-  float fr[2], c1[2], s1[2];
+  // cosines and sines of key g of the tile: pair p = 2 ks + h holds the frequencies 16 ks + 8 h + 2 t and the next
+  uint64_t cc[8], ss[8];
+  float m_run[2] = {-INFINITY, -INFINITY};   // heads 2 t and 2 t + 1
+  float l_run[2] = {0.f, 0.f};               // this lane's keys' share of the sums
+  float o[8][4];                             // dims 16 i + g and + 8, heads 2 t and 2 t + 1
 #pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    fr[i] = exp2f(-a.log2_theta * static_cast<float>(2 * (2 * lane + i)) * (1.0f / kPdDim)) * 0.31830988618379067f;
-    sincospif(fr[i], &s1[i], &c1[i]);
-  }
+  for (int i = 0; i < 8; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
 
-  float m_run = -INFINITY, l_run = 0.f;   // row g; l_run is this lane's share of the row sum
-  float o[16][4];
-#pragma unroll
-  for (int j = 0; j < 16; ++j) o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.f;
+  const int lm = lane >> 3, lr = lane & 7;
+  const uint32_t k_row = ((lm & 1) * 8 + lr) * 256, k_x = ((lm >> 1) ^ lr) << 4;             // matrices: key half, dim half
+  const uint32_t v_row = kPdTileBytes + ((lm >> 1) * 8 + lr) * 256, v_x = ((lm & 1) ^ lr) << 4;  // dim half, key half
 
   for (int j = 0; j < ntw; ++j) {
     issue(j + kPdStages - 1);
-    cp_async_wait<kPdStages - 1>();
-    __syncwarp();
     const int key0 = (tile0 + warp + j * kPdWarps) * kPdTile;
-    const uint32_t kst = ring + (j % kPdStages) * (2 * kPdTileBytes);
-    const uint32_t vst = kst + kPdTileBytes;
-    // rotate the 16 keys in place (both frequencies of the lane at once: packed fp32 pairs)
-    {
-      float cc[2], ss[2];
+    if (j % kPdReseed == 0) {
 #pragma unroll
-      for (int i = 0; i < 2; ++i) fast_sincospi(static_cast<float>(key0) * fr[i], &ss[i], &cc[i]);
-      uint64_t c2 = pack_f32x2(cc[0], cc[1]), s2 = pack_f32x2(ss[0], ss[1]);
-      const uint64_t c1p = pack_f32x2(c1[0], c1[1]), s1p = pack_f32x2(s1[0], s1[1]);
-      const uint64_t ns1p = pack_f32x2(-s1[0], -s1[1]);
-#pragma unroll
-      for (int e = 0; e < kPdTile; ++e) {
-        const uint32_t ao = kst + e * 256 + ((((lane >> 2) ^ (e & 7))) << 4) + (lane & 3) * 4;
-        uint32_t wo, wp;
-        asm volatile("ld.shared.b32 %0, [%1];\n" : "=r"(wo) : "r"(ao));
-        asm volatile("ld.shared.b32 %0, [%1];\n" : "=r"(wp) : "r"(ao + 128));
-        const float2 kof = unpack2<T>(wo), kpf = unpack2<T>(wp);
-        const uint64_t ko = pack_f32x2(kof.x, kof.y), kp = pack_f32x2(kpf.x, kpf.y);
-        const uint64_t ns2 = s2 ^ 0x8000000080000000ull;   // -s2: both sign bits flipped
-        float a0, a1, b0, b1;
-        unpack_f32x2(fma_f32x2(kp, ns2, mul_f32x2(ko, c2)), a0, a1);   // ko * c - kp * s
-        unpack_f32x2(fma_f32x2(ko, s2, mul_f32x2(kp, c2)), b0, b1);    // kp * c + ko * s
-        asm volatile("st.shared.b32 [%0], %1;\n" ::"r"(ao), "r"(pack2<T>(a0, a1)) : "memory");
-        asm volatile("st.shared.b32 [%0], %1;\n" ::"r"(ao + 128), "r"(pack2<T>(b0, b1)) : "memory");
-        const uint64_t cn = fma_f32x2(s2, ns1p, mul_f32x2(c2, c1p));   // c c1 - s s1
-        s2 = fma_f32x2(c2, s1p, mul_f32x2(s2, c1p));                   // s c1 + c s1
-        c2 = cn;
+      for (int p = 0; p < 8; ++p) {
+        const float2 f = *reinterpret_cast<const float2*>(rot + 256 + 8 * p + 2 * t);
+        const float pos = static_cast<float>(key0 + g);
+        float s0, s1, c0, c1;
+        fast_sincospi(pos * f.x, &s0, &c0);
+        fast_sincospi(pos * f.y, &s1, &c1);
+        cc[p] = pack_f32x2(c0, c1);
+        ss[p] = pack_f32x2(s0, s1);
       }
     }
+    cp_async_wait<kPdStages - 1>();
     __syncwarp();
-    // S = Q . K^T
-    // (even and odd k steps accumulate separately: two shorter chains of dependent MMAs)
-    float sc[4][4];
+    const uint32_t kst = ring + (j % kPdStages) * (2 * kPdTileBytes);
+    // S^T = K . Q^T with the keys rotated on the way (a dimension's k step and its partner's accumulate separately)
+    float sc[2][4];
 #pragma unroll
-    for (int n = 0; n < 4; ++n) sc[n][0] = sc[n][1] = sc[n][2] = sc[n][3] = 0.f;
+    for (int n = 0; n < 2; ++n) sc[n][0] = sc[n][1] = sc[n][2] = sc[n][3] = 0.f;
 #pragma unroll
-    for (int ks = 0; ks < 8; ++ks) {
-      uint32_t bf[4];
-      const int m = lane >> 3;
-      const int key = (m >> 1) * 8 + (lane & 7);
-      const int chunk = ks * 2 + (m & 1);
-      ldsm_x4(bf, kst + key * 256 + ((chunk ^ (key & 7)) << 4));
-      mma16816<T>(sc[(ks & 1) * 2], qf[ks], bf[0], bf[1]);
-      mma16816<T>(sc[(ks & 1) * 2 + 1], qf[ks], bf[2], bf[3]);
+    for (int ks = 0; ks < 4; ++ks) {
+      uint32_t own[4], par[4];
+      const uint32_t ka = kst + k_row + (k_x ^ (ks << 5));
+      ldsm_x4(own, ka);
+      ldsm_x4(par, ka + 128);
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int p = 2 * ks + h;
+        const ulonglong2 t8 = *reinterpret_cast<const ulonglong2*>(rot + 128 + (4 * p + t) * 4);
+        const ulonglong2 tw = *reinterpret_cast<const ulonglong2*>(rot + (4 * p + t) * 4);
+        uint64_t c = cc[p], s = ss[p];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {   // key g, then key g + 8
+          const float2 x = unpack2<T>(own[2 * h + e]), y = unpack2<T>(par[2 * h + e]);
+          const uint64_t ko = pack_f32x2(x.x, x.y), kp = pack_f32x2(y.x, y.y);
+          float a0, a1, b0, b1;
+          unpack_f32x2(fma_f32x2(ko, c, mul_f32x2(kp, s ^ 0x8000000080000000ull)), a0, a1);   // ko c - kp s
+          unpack_f32x2(fma_f32x2(kp, c, mul_f32x2(ko, s)), b0, b1);                           // kp c + ko s
+          own[2 * h + e] = pack2<T>(a0, a1);
+          par[2 * h + e] = pack2<T>(b0, b1);
+          if (e == 0) turn_f32x2(c, s, t8.x, t8.y);
+        }
+        turn_f32x2(cc[p], ss[p], tw.x, tw.y);
+      }
+      mma16816<T>(sc[0], own, qf[ks][0], qf[ks][1]);
+      mma16816<T>(sc[1], par, qf[ks + 4][0], qf[ks + 4][1]);
     }
-    // running softmax of row g over this lane's keys 2t, 2t+1, 8+2t, 9+2t
-    float x[4] = {sc[0][0] + sc[2][0], sc[0][1] + sc[2][1], sc[1][0] + sc[3][0], sc[1][1] + sc[3][1]};
-    const int kb = key0 + 2 * t;
-    if (kb >= seq_len) x[0] = -INFINITY;
-    if (kb + 1 >= seq_len) x[1] = -INFINITY;
-    if (kb + 8 >= seq_len) x[2] = -INFINITY;
-    if (kb + 9 >= seq_len) x[3] = -INFINITY;
-    float mx = fmaxf(fmaxf(x[0], x[1]), fmaxf(x[2], x[3]));
-    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-    const float mn = fmaxf(m_run, mx);          // finite: every tile holds at least one valid key
-    const float rescale = exp2f(m_run - mn);    // exp2f(-inf) = 0 on the first tile
+    // running softmax: keys g and g + 8 of heads 2 t and 2 t + 1
+    float x[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) x[i] = sc[0][i] + sc[1][i];
+    if (key0 + kPdTile > seq_len) {
+      if (key0 + g >= seq_len) x[0] = x[1] = -INFINITY;
+      if (key0 + g + 8 >= seq_len) x[2] = x[3] = -INFINITY;
+    }
+    float mx[2] = {fmaxf(x[0], x[2]), fmaxf(x[1], x[3])};
+    if (__any_sync(0xffffffffu, mx[0] > m_run[0] + kPdRaise || mx[1] > m_run[1] + kPdRaise)) {   // (-inf + 8 = -inf)
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+#pragma unroll
+        for (int d = 4; d < 32; d <<= 1) mx[q] = fmaxf(mx[q], __shfl_xor_sync(0xffffffffu, mx[q], d));
+        const float mn = fmaxf(m_run[q], mx[q]);
+        const float rescale = exp2f(m_run[q] - mn);   // exp2f(-inf) = 0 on the first tile
+        m_run[q] = mn;
+        l_run[q] *= rescale;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          o[i][q] *= rescale;
+          o[i][q + 2] *= rescale;
+        }
+      }
+    }
     float pr[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) pr[i] = exp2f(x[i] - mn);
-    l_run = l_run * rescale + (pr[0] + pr[1]) + (pr[2] + pr[3]);
-    m_run = mn;
+    for (int i = 0; i < 4; ++i) pr[i] = exp2f(x[i] - m_run[i & 1]);
+    l_run[0] += pr[0] + pr[2];
+    l_run[1] += pr[1] + pr[3];
+    // O^T += V^T . P^T ; P comes as [key][heads] and is transposed into the B operand
+    const uint32_t pb0 = movm_t(pack2<T>(pr[0], pr[1])), pb1 = movm_t(pack2<T>(pr[2], pr[3]));
 #pragma unroll
-    for (int jn = 0; jn < 16; ++jn) {
-      o[jn][0] *= rescale;
-      o[jn][1] *= rescale;
-    }
-    // O += P . V ; P is the A operand straight from the registers (rows 8-15 zero)
-    uint32_t pa[4] = {pack2<T>(pr[0], pr[1]), 0u, pack2<T>(pr[2], pr[3]), 0u};
-#pragma unroll
-    for (int jn = 0; jn < 16; jn += 2) {
-      uint32_t bf[4];
-      const int m = lane >> 3;
-      const int key = (m & 1) * 8 + (lane & 7);
-      const int chunk = jn + (m >> 1);
-      ldsm_x4_t(bf, vst + key * 256 + ((chunk ^ (key & 7)) << 4));
-      mma16816<T>(o[jn], pa, bf[0], bf[1]);
-      mma16816<T>(o[jn + 1], pa, bf[2], bf[3]);
+    for (int i = 0; i < 8; ++i) {
+      uint32_t vf[4];
+      ldsm_x4_t(vf, kst + v_row + ((i >> 2) << 7) + (v_x ^ ((i & 3) << 5)));
+      mma16816<T>(o[i], vf, pb0, pb1);
     }
     __syncwarp();   // the stage is free for the copy issued in the next iteration
   }
   cp_async_wait<0>();
   if (__any_sync(0xffffffffu, bad_ptr) && lane == 0 && a.err != nullptr) atomicOr(a.err, kErrBadPointer);
-  l_run += __shfl_xor_sync(0xffffffffu, l_run, 1);
-  l_run += __shfl_xor_sync(0xffffffffu, l_run, 2);
+#pragma unroll
+  for (int q = 0; q < 2; ++q)
+#pragma unroll
+    for (int d = 4; d < 32; d <<= 1) l_run[q] += __shfl_xor_sync(0xffffffffu, l_run[q], d);
   __syncthreads();   // every warp is done with its ring: it becomes the merge area
 
-  // ---- merge the warps in warp order (a fixed order): per (warp, row) m, d, 2 unused, o[128] ----
+  // ---- merge the warps in warp order (a fixed order): per (warp, head) m, l, 2 unused, o[128]; thread = dim ----
   float* red = reinterpret_cast<float*>(pd_smem);
   constexpr int REC = kPdRec;
-  float ov[32];
 #pragma unroll
-  for (int jn = 0; jn < 16; ++jn) {
-    ov[2 * jn] = o[jn][0];
-    ov[2 * jn + 1] = o[jn][1];
-  }
-  if (warp > 0) {
-    float* r = red + (warp * 8 + g) * REC;
-    if (t == 0) {
-      r[0] = m_run;
-      r[1] = l_run;
+  for (int q = 0; q < 2; ++q) {
+    const int h = 2 * t + q;
+    if (h < G) {
+      float* r = red + (warp * 8 + h) * REC;
+      if (g == 0) {
+        r[0] = m_run[q];
+        r[1] = l_run[q];
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        r[4 + 16 * i + g] = o[i][q];
+        r[4 + 16 * i + 8 + g] = o[i][q + 2];
+      }
     }
-#pragma unroll
-    for (int jn = 0; jn < 16; ++jn) *reinterpret_cast<float2*>(r + 4 + jn * 8 + 2 * t) = make_float2(ov[2 * jn], ov[2 * jn + 1]);
   }
   __syncthreads();
-  if (warp != 0) {
-    if (S == 1) return;
-  } else {
-    for (int w = 1; w < kPdWarps; ++w) {
-      const float* r = red + (w * 8 + g) * REC;
-      float o2[32];
+  T* O = static_cast<T*>(a.o) + (static_cast<size_t>(b) * Nq + head0) * kPdDim + tid;
+  float* part = a.partial + (static_cast<size_t>(b) * Nq + head0) * S * REC;   // [head][range]
 #pragma unroll
-      for (int jn = 0; jn < 16; ++jn) {
-        const float2 v2 = *reinterpret_cast<const float2*>(r + 4 + jn * 8 + 2 * t);
-        o2[2 * jn] = v2.x;
-        o2[2 * jn + 1] = v2.y;
+  for (int h = 0; h < G; ++h) {
+    float m = -INFINITY, l = 0.f, acc = 0.f;
+#pragma unroll
+    for (int w = 0; w < kPdWarps; ++w) {
+      const float* r = red + (w * 8 + h) * REC;
+      if (r[1] != 0.f) m = fmaxf(m, r[0]);   // an empty state carries no information
+    }
+#pragma unroll
+    for (int w = 0; w < kPdWarps; ++w) {
+      const float* r = red + (w * 8 + h) * REC;
+      if (r[1] != 0.f) {
+        const float wt = exp2f(r[0] - m);
+        l += r[1] * wt;
+        acc += r[4 + tid] * wt;
       }
-      pd_merge<32>(m_run, l_run, ov, r[0], r[1], o2);
+    }
+    if (ranges == 1) {
+      O[h * kPdDim] = static_cast<T>(l > 0.f ? acc * (1.0f / l) : 0.f);   // a request without keys gives zeros
+    } else {
+      float* r = part + (static_cast<size_t>(h) * S + s) * REC;
+      if (tid == 0) {
+        r[0] = m;
+        r[1] = l;
+      }
+      r[4 + tid] = acc;
     }
   }
+  if (ranges == 1) return;
 
-  T* O = static_cast<T*>(a.o);
-  auto store_out = [&]() {   // warp 0: row g = head, this lane's 32 columns
-    if (g >= G) return;
-    const float inv = l_run > 0.f ? 1.0f / l_run : 0.f;   // a request without keys gives zeros
-    T* op = O + (static_cast<size_t>(b) * Nq + head0 + g) * kPdDim;
-#pragma unroll
-    for (int jn = 0; jn < 16; ++jn)
-      *reinterpret_cast<uint32_t*>(op + jn * 8 + 2 * t) = pack2<T>(ov[2 * jn] * inv, ov[2 * jn + 1] * inv);
-  };
-
-  if (S == 1) {
-    if (warp == 0) store_out();
-    return;
-  }
-
-  // ---- several ranges: park the partial state, the last CTA of the (request, kv head) merges ----
-  if (warp == 0 && g < G) {
-    float* r = a.partial + ((static_cast<size_t>(b) * Nq + head0 + g) * S + s) * REC;
-    if (t == 0) {
-      r[0] = m_run;
-      r[1] = l_run;
-    }
-#pragma unroll
-    for (int jn = 0; jn < 16; ++jn) *reinterpret_cast<float2*>(r + 4 + jn * 8 + 2 * t) = make_float2(ov[2 * jn], ov[2 * jn + 1]);
-    __threadfence();
-  }
+  // ---- several ranges: the last CTA of the (request, kv head) merges the parked states in range order ----
+  __threadfence();
   __syncthreads();
   if (tid == 0) {
     const int old = atomicAdd(a.tickets + bh, 1);
-    s_last = old == S - 1;
-    if (old == S - 1) a.tickets[bh] = 0;   // leave the workspace ready for the next launch
+    s_last = old == ranges - 1;
+    if (old == ranges - 1) a.tickets[bh] = 0;   // leave the workspace ready for the next launch
   }
   __syncthreads();
-  if (!s_last || warp != 0 || g >= G) return;
+  if (!s_last) return;
   __threadfence();
-  m_run = -INFINITY;
-  l_run = 0.f;
+#pragma unroll 1
+  for (int h = 0; h < G; ++h) {
+    const float* r0 = part + static_cast<size_t>(h) * S * REC;
+    float mz[kPdMaxSplits], lz[kPdMaxSplits], oz[kPdMaxSplits];
+    float m = -INFINITY, l = 0.f, acc = 0.f;
 #pragma unroll
-  for (int i = 0; i < 32; ++i) ov[i] = 0.f;
-  for (int z = 0; z < S; ++z) {
-    const float* r = a.partial + ((static_cast<size_t>(b) * Nq + head0 + g) * S + z) * REC;
-    const float m2 = __ldcg(r), d2 = __ldcg(r + 1);
-    float o2[32];
-#pragma unroll
-    for (int jn = 0; jn < 16; ++jn) {
-      const float2 v2 = __ldcg(reinterpret_cast<const float2*>(r + 4 + jn * 8 + 2 * t));
-      o2[2 * jn] = v2.x;
-      o2[2 * jn + 1] = v2.y;
+    for (int z = 0; z < kPdMaxSplits; ++z) {
+      mz[z] = lz[z] = oz[z] = 0.f;
+      if (z < ranges) {
+        mz[z] = __ldcg(r0 + z * REC);
+        lz[z] = __ldcg(r0 + z * REC + 1);
+        oz[z] = __ldcg(r0 + z * REC + 4 + tid);
+      }
     }
-    pd_merge<32>(m_run, l_run, ov, m2, d2, o2);
+#pragma unroll
+    for (int z = 0; z < kPdMaxSplits; ++z)
+      if (lz[z] != 0.f) m = fmaxf(m, mz[z]);
+#pragma unroll
+    for (int z = 0; z < kPdMaxSplits; ++z) {
+      if (lz[z] != 0.f) {
+        const float wt = exp2f(mz[z] - m);
+        l += lz[z] * wt;
+        acc += oz[z] * wt;
+      }
+    }
+    O[h * kPdDim] = static_cast<T>(l > 0.f ? acc * (1.0f / l) : 0.f);
   }
-  store_out();
 }
 
 }  // namespace smlm

@@ -631,11 +631,18 @@ int launch_rms_bwd(void* dx, void* dw, const void* go, const void* x, const void
 }
 
 // ---- paged key-value cache ----------------------------------------------------------
-// Page ranges a (request, kv head) is cut into, so that small batches still fill the machine.  The
+// Page ranges a (request, kv head) is cut into at most, so that small batches still fill the machine.  The
 // sequence lengths live on the device, so the choice depends on the batch shape only.
 inline int decode_splits(int batch, int num_kv_heads) {
   const int ctas = std::max(1, batch * num_kv_heads);
   return std::max(1, std::min(kPdMaxSplits, (3 * kNumSMs + ctas - 1) / ctas));
+}
+
+// The shortest range worth a CTA: what an even share of the batch's tiles (the pages bound them from above) would
+// be, but no more than 32 tiles (8 per warp cover a CTA's set-up) and a tile per warp at least.
+inline int decode_min_tiles(int total_pages, int page_size, int num_kv_heads) {
+  const long long tiles = static_cast<long long>(total_pages) * page_size / kPdTile * num_kv_heads;
+  return static_cast<int>(std::max<long long>(kPdWarps, std::min<long long>(32, tiles / (3 * kNumSMs))));
 }
 
 inline size_t decode_ticket_bytes(int batch, int num_kv_heads) {
@@ -1168,6 +1175,9 @@ int smlm_b200_batch_decode(void* o, const void* q, const void* const* kv_ptrs, c
                                                               decode_ticket_bytes(batch_size, num_kv_heads));
   a.batch = batch_size; a.num_kv_heads = num_kv_heads; a.num_layers = num_layers; a.layer_idx = layer_idx;
   a.page_size = page_size; a.total_pages = total_pages;
+  a.min_tiles = decode_min_tiles(total_pages, page_size, num_kv_heads);
+  // longest requests first where the CTAs take more than one round and the ranks are cheap to find
+  a.sorted = a.splits == 1 && batch_size <= kPdMaxSorted && batch_size * num_kv_heads > 3 * kNumSMs ? 1 : 0;
   a.log2_theta = std::log2(rope_theta);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   return dtype == SMLM_F16 ? dispatch_decode<__half>(a, group, st) : dispatch_decode<__nv_bfloat16>(a, group, st);

@@ -1,0 +1,59 @@
+"""Decode attention at the sizes where its tiles and ranges end.  Tolerance: keys, softmax weights
+and results are rounded to 16 bits once each (2^-9 relative in bf16), scores and sums are fp32; three such roundings of
+values of order one stay below rtol = atol = 1e-2."""
+import numpy as np
+import pytest
+import torch
+
+from helpers import assert_close
+from oracle import attention_oracle as A
+
+pytestmark = pytest.mark.gpu
+DEV = torch.device("cuda:0")
+THETA = 10000.0
+
+
+def _cache(seed, seqlens, N, P, dtype):
+    pages, indptr, last = A.make_cache(seed, seqlens, 1, N, P, 128, dtype)
+    pd = [p.to(DEV).contiguous() for p in pages]
+    dev = dict(keep=pd, ptrs=torch.tensor([p.data_ptr() for p in pd], dtype=torch.int64, device=DEV),
+               ind=torch.tensor(indptr, dtype=torch.int32, device=DEV),
+               last=torch.tensor(last, dtype=torch.int32, device=DEV))
+    return (pages, indptr, last), dev
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("group,batch", [(1, 3), (4, 3), (8, 2), (4, 60), (2, 65), (8, 57)])
+def test_decode_at_the_edges_of_tiles_ranges_and_ranks(dtype, group, batch):
+    """Tiles of 16 keys, a warp's step of 64, the rotation computed afresh every 1024 keys; small batches are cut into
+    ranges, from 56 requests of 8 heads on the requests go by length: equal lengths, empty requests and a last
+    request among them, batches that are no multiple of four."""
+    from loquetier_b200 import kvcache
+    N, P = 8, 16
+    edge = [1023, 1024, 1025, 2100, 15, 16, 17, 63, 64, 65, 0, 1, 128, 129, 64, 0, 17]
+    seqlens = (edge * 4)[:batch] if batch > 3 else [1025, 2100, 17][:batch]
+    host, d = _cache(50 + group + batch, seqlens, N, P, dtype)
+    q = torch.randn((batch, N * group, 128), generator=torch.Generator().manual_seed(batch)).to(dtype)
+    outs = []
+    for _ in range(2):
+        o = torch.full(q.shape, float("nan"), dtype=dtype, device=DEV)
+        word = torch.zeros(1, dtype=torch.int32, device=DEV)
+        kvcache.batch_decode_into(o, q.to(DEV), d["ptrs"], d["ind"], d["last"], 1, 0, N, THETA, P, status_word=word)
+        assert int(word.item()) == 0
+        outs.append(o)
+    assert torch.equal(outs[0], outs[1])   # merged in a fixed order
+    assert_close(outs[0], A.batch_decode(q, *host, 0, THETA), what=f"group {group} batch {batch}")
+
+
+def test_decode_scores_that_grow_along_the_sequence():
+    """Keys scaled up with their position: the maxima are raised again and again, in every warp and range."""
+    from loquetier_b200 import kvcache
+    N, group, P, L = 1, 4, 16, 900
+    (pages, indptr, last), d = _cache(77, [L], N, P, torch.float16)
+    for i, pg in enumerate(pages):
+        pg[:, 0] *= 1.0 + 0.1 * i
+        d["keep"][i].copy_(pg)
+    q = (torch.randn((1, group, 128), generator=torch.Generator().manual_seed(78)) * 1.5).to(torch.float16)
+    o = torch.empty(q.shape, dtype=q.dtype, device=DEV)
+    kvcache.batch_decode_into(o, q.to(DEV), d["ptrs"], d["ind"], d["last"], 1, 0, N, THETA, P)
+    assert_close(o, A.batch_decode(q, pages, indptr, last, 0, THETA), what="raised maxima")
