@@ -66,6 +66,12 @@ size_t smlm_b200_tmp_size(int num_problems);
  * reference only gets from a batch sorted by adapter.  nseg <= 4096 for the grouped plan to apply. */
 int smlm_b200_group_ids_from_pointers(const void* const* w_table, int nseg, int32_t* ids_out, void* stream);
 
+/* Writes `bytes` (a multiple of 4) from host memory to device memory through kernel parameters: no staging copy,
+ * no wait for the stream, and the host buffer may be reused on return.  For the small arrays of a call - pointer
+ * tables, adapter ids, index pointers (3.5 KB per launch).  Stream-ordered; can be captured in a CUDA graph, which
+ * then replays the values of the time of capture. */
+int smlm_b200_upload(void* dst, const void* host, size_t bytes, void* stream);
+
 /* Segment bookkeeping on the device: the run-length merge of the ordered requests of a step into
  * segments, bit-identical to the reference's host loop (src/loquetier_src/model_generation.py:267-283:
  * neighbours with the same adapter become one segment; `segment` = cumsum of the lengths with a
@@ -175,8 +181,10 @@ int smlm_b200_fwd(void* y, const void* x, void* v, const void* const* wa_table, 
  * next call's shape (T, npart, rank, column counts, or the kinds selected by
  * smlm_b200_wgrad_select_multi) differs from the previous call's on the same workspace:
  * a different shape puts the boundary between tickets and parked sums elsewhere, and what
- * one shape parked lies where another expects tickets.  Launches that overlap in time must
+ * one shape parked lies where another expects tickets.  Not needed between two shapes whose heads both have the
+ * smallest size, SMLM_TICKET_HEAD bytes: their boundary is the same.  Launches that overlap in time must
  * not share a workspace. */
+#define SMLM_TICKET_HEAD 65536
 size_t smlm_b200_wgrad_workspace_bytes(int T, int npart, int rank, int h0, int h1);
 size_t smlm_b200_wgrad_ticket_bytes(int T, int npart, int rank, int h0, int h1);
 

@@ -6,6 +6,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cmath>
+#include <cstring>
 #include <mutex>
 #include <utility>
 #include <vector>
@@ -413,10 +414,15 @@ inline int wgrad_rt(int R) {
   return rtb > 4 ? 8 : (rtb > 2 ? 4 : rtb);
 }
 
+// Head of a workspace that holds `bytes` of tickets.  Nearly every shape needs less than 64 KB, so a workspace
+// that serves calls of different shapes keeps its boundary between tickets and parked sums, and the tickets
+// that every launch leaves zeroed stay valid: its owner need not clear them in between.
+inline size_t ticket_head(size_t bytes) { return std::max<size_t>(SMLM_TICKET_HEAD, (bytes + 255) / 256 * 256); }
+
 // How a batch of T token rows in npart partitions is cut for the jobs' column counts.
 struct WgradShape {
   int slab, slabs_total, group, groups;
-  size_t ticket_bytes, scratch_bytes;
+  size_t tickets_used, ticket_bytes, scratch_bytes;   // ticket_bytes: the head that holds them
 };
 
 // The tcgen05 variant serves every rank above 32 unless it is switched off, and the lower ranks
@@ -451,7 +457,8 @@ WgradShape wgrad_shape(int T, int npart, int R, const int* h, int nh, bool tc) {
   }
   s.group = static_cast<int>(g);
   s.groups = (mp + s.group - 1) / s.group;
-  s.ticket_bytes = (static_cast<size_t>(npart) * s.slabs_total * 4 * sizeof(int) + 255) / 256 * 256;
+  s.tickets_used = (static_cast<size_t>(npart) * s.slabs_total * 4 * sizeof(int) + 255) / 256 * 256;
+  s.ticket_bytes = ticket_head(s.tickets_used);
   s.scratch_bytes = static_cast<size_t>(s.groups) * 2 * s.slabs_total * (rt * 16) * s.slab * sizeof(float);
   return s;
 }
@@ -540,8 +547,9 @@ size_t wgrad_ticket_need(int T, int npart, int R, const int* h, int nh) {
 // is handed buffers but owns no allocator, or under a framework whose memory pool must
 // not be bypassed.  For them the weight-gradient kernel's workspace lives in this fixed
 // array in the library's own device image.  Every GPU that loads the library carries the
-// array (kStaticWgradBytes) until the process exits.
-constexpr size_t kStaticWgradBytes = SMLM_STATIC_WGRAD_BYTES;
+// array (kStaticWgradBytes) until the process exits.  The limit of a call counts the tickets it uses; the array
+// has room for the smallest head on top.
+constexpr size_t kStaticWgradBytes = SMLM_STATIC_WGRAD_BYTES + SMLM_TICKET_HEAD;
 static __device__ __align__(256) unsigned char g_wgrad_static_scratch[kStaticWgradBytes];
 
 std::mutex g_static_mutex;
@@ -646,7 +654,7 @@ inline int decode_min_tiles(int total_pages, int page_size, int num_kv_heads) {
 }
 
 inline size_t decode_ticket_bytes(int batch, int num_kv_heads) {
-  return (static_cast<size_t>(batch) * num_kv_heads * sizeof(int) + 255) / 256 * 256;
+  return ticket_head(static_cast<size_t>(batch) * num_kv_heads * sizeof(int));
 }
 
 template <typename T, int G>
@@ -822,6 +830,34 @@ int smlm_b200_merge_segments(const int32_t* req_ids, const int32_t* req_len, int
   return SMLM_OK;
 }
 
+int smlm_b200_upload(void* dst, const void* host, size_t bytes, void* stream) {
+  if (bytes == 0) return SMLM_OK;
+  if (dst == nullptr || host == nullptr || (bytes & 3) != 0) return SMLM_ERR_INVALID_ARGUMENT;
+  if ((reinterpret_cast<uintptr_t>(dst) & 3) != 0) return SMLM_ERR_MISALIGNED;
+  // 512 bytes cover the tables of one projection; 3.5 KB stay under the parameter limit of every toolkit
+  constexpr int kSmall = 128, kLarge = 896;
+  uint32_t* d = static_cast<uint32_t*>(dst);
+  const char* h = static_cast<const char*>(host);
+  for (size_t left = bytes / 4; left > 0;) {
+    const int n = static_cast<int>(std::min<size_t>(left, left <= kSmall ? kSmall : kLarge));
+    int rc;
+    if (n <= kSmall) {
+      UploadWords<kSmall> u;
+      std::memcpy(u.w, h, n * 4);
+      rc = launch(upload_kernel<kSmall>, dim3(1, 1, 1), kUploadThreads, 1, 0, static_cast<cudaStream_t>(stream), d, n, u);
+    } else {
+      UploadWords<kLarge> u;
+      std::memcpy(u.w, h, n * 4);
+      rc = launch(upload_kernel<kLarge>, dim3(1, 1, 1), kUploadThreads, 1, 0, static_cast<cudaStream_t>(stream), d, n, u);
+    }
+    if (rc != SMLM_OK) return rc;
+    d += n;
+    h += static_cast<size_t>(n) * 4;
+    left -= n;
+  }
+  return SMLM_OK;
+}
+
 int smlm_b200_group_ids_from_pointers(const void* const* w_table, int nseg, int32_t* ids_out, void* stream) {
   if (nseg < 0) return SMLM_ERR_INVALID_ARGUMENT;
   if (nseg == 0) return SMLM_OK;
@@ -942,7 +978,7 @@ int smlm_b200_wgrad_static(void* const* g_table, const void* p, const void* q, c
   // launch all follow this one reading of the process-wide mode
   const bool tc = wgrad_uses_tensor_cores(rank);
   const WgradShape sh = wgrad_shape(T, npart, rank, &h, 1, tc);
-  if (sh.ticket_bytes + sh.scratch_bytes > kStaticWgradBytes) return SMLM_ERR_STATIC_LIMIT;
+  if (sh.tickets_used + sh.scratch_bytes > SMLM_STATIC_WGRAD_BYTES) return SMLM_ERR_STATIC_LIMIT;
   void* scratch = nullptr;
   const int rc = static_scratch_of_current_device(&scratch);
   if (rc != SMLM_OK) return rc;

@@ -64,7 +64,15 @@ class BatchLenInfo:
 
 
 def _ptr_table(tensors: Sequence[torch.Tensor], device) -> torch.Tensor:
-    return torch.tensor([t.data_ptr() for t in tensors], dtype=torch.int64, device=device)
+    return ops.device_ints([t.data_ptr() for t in tensors], torch.int64, device)
+
+
+def _ptr_tables(groups: Sequence[Sequence[torch.Tensor]], device) -> Tuple[torch.Tensor, ...]:
+    """One pointer table per group of tensors (all of one length), from a single upload."""
+    n = len(groups[0])
+    if n == 0:
+        return tuple(_ptr_table(g, device) for g in groups)
+    return _ptr_table([t for g in groups for t in g], device).split(n)
 
 
 class add_lora(Function):
@@ -111,13 +119,13 @@ class add_lora(Function):
         if tl == 0:
             return (None, grad_x, None, None, None, None, None, None,
                     *[torch.zeros_like(w) for w in weight_list])
-        part = torch.tensor([int(t) for t in tp[:npart + 1]], dtype=torch.int32, device=dev)
+        part = ops.device_ints([int(t) for t in tp[:npart + 1]], torch.int32, dev)
         plan = ops.Plan(part, tl)
         was, wbs = weight_list[0:2 * npart:2], weight_list[1:2 * npart:2]
         grads = [torch.empty_like(w) for w in weight_list[:2 * npart]]
         dv = torch.empty((tl, ctx.rank), dtype=go.dtype, device=dev)
-        ops.bwd(grad_x, _ptr_table(grads[::2], dev), _ptr_table(grads[1::2], dev), dv, go,
-                x.contiguous(), v.contiguous(), _ptr_table(was, dev), _ptr_table(wbs, dev), plan, ctx.rank,
+        dA_t, dB_t, wa_t, wb_t = _ptr_tables((grads[::2], grads[1::2], was, wbs), dev)
+        ops.bwd(grad_x, dA_t, dB_t, dv, go, x.contiguous(), v.contiguous(), wa_t, wb_t, plan, ctx.rank,
                 is_row_major=False)
         grads += [None] * (len(weight_list) - 2 * npart)
         return None, grad_x, None, None, None, None, None, None, *grads

@@ -54,9 +54,8 @@ def smlm_forward_cutlass(y: torch.Tensor, x: torch.Tensor, w_ptr: torch.Tensor, 
         # indices are derived on the device and a grouped plan gathers each adapter's decode tokens into one
         # piece, so that its panel is fetched once - sorted batch or not.  Nothing is read back to the host.
         ids = torch.empty(nseg, dtype=torch.int32, device=x.device)
-        with torch.cuda.device(x.device):
-            ops.check(lib.smlm_b200_group_ids_from_pointers(w_ptr.data_ptr(), nseg, ids.data_ptr(),
-                                                            torch.cuda.current_stream(x.device).cuda_stream),
+        with ops.on_device(x):
+            ops.check(lib.smlm_b200_group_ids_from_pointers(w_ptr.data_ptr(), nseg, ids.data_ptr(), ops._stream(x)),
                       "smlm_b200_group_ids_from_pointers")
         plan = ops.Plan(s, T, seg_ids=ids, n_table=nseg)
         ops.gemm(y, x, w_ptr[:nseg], plan, is_row_major=bool(is_row_major), seg_ids=ids)

@@ -17,6 +17,7 @@ import torch
 
 from . import cabi
 from .cabi import check, lib
+from .ops import _stream, on_device
 
 _DT = {torch.float16: cabi.SMLM_F16, torch.bfloat16: cabi.SMLM_BF16}
 
@@ -153,11 +154,7 @@ class BatchedKvCache:
 # ---------------------------------------------------------------------------
 
 _WORKSPACES = {}
-_WS_SHAPE = {}
-
-
-def _stream(t):
-    return torch.cuda.current_stream(t.device).cuda_stream
+_WS_HEAD = {}   # device -> bytes of tickets at the head of the workspace for the batch it last served
 
 
 def _dtype_code(t):
@@ -169,28 +166,27 @@ def _dtype_code(t):
 
 def decode_workspace(device, batch: int, num_qo_heads: int, num_kv_heads: int) -> Optional[torch.Tensor]:
     """Scratch of the decode kernel with its tickets zeroed, cached per device and grown on demand.  The kernel
-    leaves the tickets zeroed, but another batch shape moves the boundary between tickets and parked softmax
-    states, so the head is cleared again whenever the shape differs from the previous one.  Ask for it right
-    before the launch; calls that may overlap on different streams need workspaces of their own."""
+    leaves the tickets zeroed; a batch whose tickets take another head moves the boundary between tickets and
+    parked softmax states, so the head is cleared then.  Ask for it right before the launch; calls that may
+    overlap on different streams need workspaces of their own."""
     shape = (int(batch), int(num_qo_heads), int(num_kv_heads))
     need = int(lib.smlm_b200_batch_decode_workspace_bytes(*shape))
+    head = int(lib.smlm_b200_batch_decode_ticket_bytes(shape[0], shape[2]))
     ws = _WORKSPACES.get(device)
     if ws is None or ws.numel() < need:
         ws = torch.zeros(max(need, 1 << 16), dtype=torch.uint8, device=device)
         _WORKSPACES[device] = ws
-    elif _WS_SHAPE.get(device) != shape:
-        tickets = int(lib.smlm_b200_batch_decode_ticket_bytes(int(batch), int(num_kv_heads)))
-        if tickets > 0:
-            with torch.cuda.device(device):
-                ws[:tickets].zero_()
-    _WS_SHAPE[device] = shape
+    elif _WS_HEAD.get(device) != head and head > 0:
+        with on_device(ws):
+            ws[:head].zero_()
+    _WS_HEAD[device] = head
     return ws
 
 
 def batch_decode_into(o, q, kv_ptrs, kv_indptr, last_page_offset, num_layers, layer_idx, num_kv_heads, base, page_size,
                       workspace=None, status_word=None):
     ws = workspace if workspace is not None else decode_workspace(q.device, q.size(0), q.size(1), num_kv_heads)
-    with torch.cuda.device(q.device):
+    with on_device(q):
         check(lib.smlm_b200_batch_decode(o.data_ptr(), q.data_ptr(), kv_ptrs.data_ptr(), kv_indptr.data_ptr(),
                                          last_page_offset.data_ptr(), ws.data_ptr(), ws.numel(),
                                          None if status_word is None else status_word.data_ptr(),
@@ -227,7 +223,7 @@ def batch_prefill_into(o, q, qo_indptr, kv_ptrs, kv_indptr, last_page_offset, nu
                        base, page_size, workspace=None, status_word=None):
     ws = workspace if workspace is not None else prefill_workspace(q.device, kv_ptrs.numel(), page_size,
                                                                    num_kv_heads)
-    with torch.cuda.device(q.device):
+    with on_device(q):
         check(lib.smlm_b200_batch_prefill(o.data_ptr(), q.data_ptr(), qo_indptr.data_ptr(), kv_ptrs.data_ptr(),
                                           kv_indptr.data_ptr(), last_page_offset.data_ptr(), ws.data_ptr(),
                                           ws.numel(), None if status_word is None else status_word.data_ptr(),
@@ -252,7 +248,7 @@ def batch_prefill(q: torch.Tensor, qo_indptr: torch.Tensor, kv: BatchedKvCache, 
 
 def init_kv_raw(kv_ptrs, kv_indptr, last_page_offset, k, v, seqlen_indptr, num_layers, layer_idx, num_kv_heads,
                 page_size, status_word=None):
-    with torch.cuda.device(k.device):
+    with on_device(k):
         check(lib.smlm_b200_init_kv(kv_ptrs.data_ptr(), kv_indptr.data_ptr(), last_page_offset.data_ptr(),
                                     k.data_ptr(), v.data_ptr(), seqlen_indptr.data_ptr(),
                                     None if status_word is None else status_word.data_ptr(),
@@ -270,7 +266,7 @@ def init_kv(kv: BatchedKvCache, k: torch.Tensor, v: torch.Tensor, seqlen_indptr:
 
 def append_kv_raw(kv_ptrs, kv_indptr, last_page_offset, k, v, num_layers, layer_idx, num_kv_heads, page_size,
                   status_word=None):
-    with torch.cuda.device(k.device):
+    with on_device(k):
         check(lib.smlm_b200_append_kv(kv_ptrs.data_ptr(), kv_indptr.data_ptr(), last_page_offset.data_ptr(),
                                       k.data_ptr(), v.data_ptr(),
                                       None if status_word is None else status_word.data_ptr(), int(k.size(0)),

@@ -18,7 +18,7 @@ from torch import nn
 from torch.autograd.function import Function
 
 from . import ops
-from .kernel_utils import BatchLenInfo, _ptr_table, add_lora
+from .kernel_utils import BatchLenInfo, _ptr_table, _ptr_tables, add_lora
 from .segments import wants_grouped_plan
 
 
@@ -57,24 +57,28 @@ class MixedLoraContext:
         st = self._dev.get(key)
         if st is None:
             seg = self._segment.to(device=device, dtype=torch.int32).contiguous()
-            seg_ids = torch.tensor(list(self._lora_ids), dtype=torch.int32, device=device)
+            ids = list(self._lora_ids)
+            seg_ids = ops.device_ints(ids, torch.int32, device)
             # grouped plan when it helps: decode tokens of one adapter then share its panels wherever they
-            # sit in the batch.  The reference keeps `segment` on the device (model_generation.py:279-283):
-            # its lengths come back in ONE copy, outside any stream capture (the state is built on the
-            # first forward after `update`), never element by element.
-            bounds = self._segment.tolist()
-            lens = [b - a for a, b in zip(bounds[:-1], bounds[1:])]
-            if wants_grouped_plan(lens, list(self._lora_ids)):
-                plan = ops.Plan(seg, T, seg_ids=seg_ids, n_table=max(self._lora_ids) + 1)
-            else:
-                plan = ops.Plan(seg, T)
-            st = dict(segment=seg, plan=plan, seg_ids=seg_ids)
+            # sit in the batch.  Only an adapter with several segments can ask for it; then the segments' lengths
+            # are needed.  The reference keeps `segment` on the device (model_generation.py:279-283): they come
+            # back in ONE copy, outside any stream capture (the state is built on the first forward after
+            # `update`), never element by element.
+            grouped = False
+            if len(set(ids)) < len(ids):
+                bounds = self._segment.tolist()
+                grouped = wants_grouped_plan([b - a for a, b in zip(bounds[:-1], bounds[1:])], ids)
             tl = int(self._blen.tlen) if self._blen is not None else 0
+            group = dict(seg_ids=seg_ids, n_table=max(ids) + 1) if grouped else {}
             if tl > 0:
                 tp = [int(v) for v in self._blen.train_partition]
-                part = torch.tensor(tp, dtype=torch.int32, device=device)
-                st.update(part=part, part_plan=ops.Plan(part, tl), tlen=tl,
-                          part_ids=torch.tensor(list(self._train_idx), dtype=torch.int32, device=device))
+                part = ops.device_ints(tp, torch.int32, device)
+                plan, part_plan = ops.plan_pair(seg, T, part, tl, seg_ids_a=group.get("seg_ids"),
+                                                n_table_a=group.get("n_table", 0))
+                st = dict(segment=seg, plan=plan, seg_ids=seg_ids, part=part, part_plan=part_plan, tlen=tl,
+                          part_ids=ops.device_ints(list(self._train_idx), torch.int32, device))
+            else:
+                st = dict(segment=seg, plan=ops.Plan(seg, T, **group), seg_ids=seg_ids)
             self._dev[key] = st
         return st
 
@@ -132,9 +136,9 @@ class _lora_linear_fn(Function):
             dA = [torch.empty_like(mod.adapters[i].wa) for i in mod.root_context.train_idx[:npart]]
             dB = [torch.empty_like(mod.adapters[i].wb) for i in mod.root_context.train_idx[:npart]]
             dv = torch.empty((tl, mod.rank), dtype=go.dtype, device=go.device)
-            ops.bwd(grad_x, _ptr_table(dA, go.device), _ptr_table(dB, go.device), dv, go, x.contiguous(),
-                    v.contiguous(), mod.wa_ptrs, mod.wb_ptrs, st["part_plan"], mod.rank, is_row_major=False,
-                    part_ids=st["part_ids"], part_scale=mod.scaling_f32)
+            dA_t, dB_t = _ptr_tables((dA, dB), go.device)
+            ops.bwd(grad_x, dA_t, dB_t, dv, go, x.contiguous(), v.contiguous(), mod.wa_ptrs, mod.wb_ptrs,
+                    st["part_plan"], mod.rank, is_row_major=False, part_ids=st["part_ids"], part_scale=mod.scaling_f32)
             grads = [g for pair in zip(dA, dB) for g in pair]
         return (grad_out, grad_x, None, None, *grads)
 

@@ -3,6 +3,7 @@ sizes and the current CUDA stream.  Device memory (outputs, the plan buffer) is
 allocated by torch; the library itself never allocates and never synchronises."""
 from __future__ import annotations
 
+import array
 from typing import Optional
 
 import torch
@@ -22,7 +23,44 @@ def _dtype_code(t: torch.Tensor) -> int:
 
 
 def _stream(t: torch.Tensor) -> int:
-    return torch.cuda.current_stream(t.device).cuda_stream
+    """The current stream of the tensor's device as the driver's handle (no Stream object is made)."""
+    return torch._C._cuda_getCurrentRawStream(t.get_device())
+
+
+class _SameDevice:
+    """Stands in for ``torch.cuda.device`` where the device is the current one already."""
+
+    def __enter__(self):
+        return None
+
+    def __exit__(self, *exc):
+        return False
+
+
+_SAME_DEVICE = _SameDevice()
+
+
+def on_device(t: torch.Tensor):
+    """``torch.cuda.device(t.device)``, without the switch where nothing changes."""
+    i = t.get_device()
+    return _SAME_DEVICE if i >= 0 and i == torch.cuda.current_device() else torch.cuda.device(t.device)
+
+
+_UPLOAD_LIMIT = 1 << 14   # bytes; above, one pageable copy costs less than the launches
+
+
+def device_ints(values, dtype: torch.dtype, device) -> torch.Tensor:
+    """``torch.tensor(values, dtype, device=device)`` for int32 / int64, written by a launch that carries the values
+    in its parameters: the host does not wait for the stream as it does for a copy from pageable memory."""
+    device = torch.device(device)
+    if device.type != "cuda" or not 0 < len(values) <= _UPLOAD_LIMIT // 8:
+        return torch.tensor(values, dtype=dtype, device=device)
+    host = array.array("q" if dtype == torch.int64 else "i", values)
+    t = torch.empty(len(host), dtype=dtype, device=device)
+    with on_device(t):
+        check(lib.smlm_b200_upload(t.data_ptr(), host.buffer_info()[0], len(host) * host.itemsize, _stream(t)),
+              "smlm_b200_upload")
+    return t
 
 
 def _p(t: Optional[torch.Tensor]):
@@ -67,7 +105,7 @@ class Plan:
         self.nbytes = nbytes
         if not launch:
             return
-        with torch.cuda.device(indptr.device):
+        with on_device(indptr):
             check(lib.smlm_b200_plan_grouped(self.buf.data_ptr(), nbytes, indptr.data_ptr(), _p(seg_ids), self.nseg,
                                              self.n_table, self.T, _stream(indptr)), "smlm_b200_plan")
 
@@ -75,7 +113,7 @@ class Plan:
         """Synchronises.  Returns (n_pieces, status code)."""
         import ctypes
         n = ctypes.c_int(0)
-        with torch.cuda.device(self.buf.device):
+        with on_device(self.buf):
             rc = lib.smlm_b200_plan_status(self.buf.data_ptr(), ctypes.byref(n), _stream(self.buf))
         return n.value, rc
 
@@ -90,7 +128,7 @@ def plan_pair(indptr_a: torch.Tensor, T_a: int, indptr_b: torch.Tensor, T_b: int
     partitions - built by one launch.  Returns (plan_a, plan_b)."""
     a = Plan(indptr_a, T_a, seg_ids=seg_ids_a, n_table=n_table_a, launch=False)
     b = Plan(indptr_b, T_b, launch=False)
-    with torch.cuda.device(indptr_a.device):
+    with on_device(indptr_a):
         check(lib.smlm_b200_plan_pair(a.buf.data_ptr(), a.nbytes, indptr_a.data_ptr(), _p(seg_ids_a), a.nseg,
                                       a.n_table, a.T, b.buf.data_ptr(), b.nbytes, indptr_b.data_ptr(), b.nseg, b.T,
                                       _stream(indptr_a)), "smlm_b200_plan_pair")
@@ -111,7 +149,7 @@ def set_cluster_split(split: int) -> int:
 
 def gemm(y, x, w_table, plan: Plan, is_row_major=False, seg_ids=None, seg_scale=None, accumulate=False):
     """One segmented GEMM (one reference operator call)."""
-    with torch.cuda.device(x.device):
+    with on_device(x):
         check(lib.smlm_b200_gemm(y.data_ptr(), x.data_ptr(), w_table.data_ptr(), _p(seg_ids), _p(seg_scale),
                                  plan.buf.data_ptr(), int(w_table.numel()), int(x.size(0)), plan.nseg,
                                  int(x.size(1)), int(y.size(1)), _dtype_code(x), int(bool(is_row_major)),
@@ -129,7 +167,7 @@ def fwd(y, x, v, wa_table, wb_table, plan: Plan, rank: int, is_row_major=False, 
     and may run alongside all of them (its read phase overlaps their write phases); it still
     completes after them.  A call that consumes the output of an earlier launch must therefore pass
     ``independent=False`` even when unrelated independent launches sit between the two."""
-    with torch.cuda.device(x.device):
+    with on_device(x):
         check(lib.smlm_b200_fwd(y.data_ptr(), x.data_ptr(), v.data_ptr(), wa_table.data_ptr(),
                                 wb_table.data_ptr(), _p(seg_ids), _p(seg_scale), plan.buf.data_ptr(),
                                 int(wa_table.numel()), int(x.size(0)), plan.nseg, int(x.size(1)),
@@ -142,7 +180,7 @@ def fwd(y, x, v, wa_table, wb_table, plan: Plan, rank: int, is_row_major=False, 
 def bwd_dx(dx, dv, go, wa_table, wb_table, plan: Plan, rank: int, is_row_major=False, part_ids=None,
            part_scale=None, independent=False):
     """dV = scale * gO . B and dX = dV . A over the train partitions of ``plan``."""
-    with torch.cuda.device(go.device):
+    with on_device(go):
         check(lib.smlm_b200_bwd_dx(dx.data_ptr(), dv.data_ptr(), go.data_ptr(), wa_table.data_ptr(),
                                    wb_table.data_ptr(), _p(part_ids), _p(part_scale), plan.buf.data_ptr(),
                                    int(wa_table.numel()), plan.T, plan.nseg, int(dx.size(1)), int(go.size(1)),
@@ -154,23 +192,25 @@ def bwd_dx(dx, dv, go, wa_table, wb_table, plan: Plan, rank: int, is_row_major=F
 _WORKSPACES = {}
 
 
-_WS_SHAPE = {}   # (device, slot) -> the shape the cached workspace was last handed out for
+_WS_SHAPE = {}   # (device, slot) -> (shape, bytes of tickets) the cached workspace was last handed out for
 
 
 def _cached_workspace(device, slot, need: int, shape, ticket_bytes: int) -> torch.Tensor:
     """One buffer per (device, slot), grown on demand and zero-filled when (re)allocated.  The kernels leave
-    the tickets at its head zeroed, but a different shape moves the boundary between tickets and parked sums,
-    so the head is cleared again (a few KB, on the current stream) whenever the shape differs from the one the
-    buffer was last handed out for."""
+    the tickets at its head zeroed.  As long as every shape's tickets fit the smallest head the boundary between
+    tickets and parked sums stands still; where a shape needs more, it moves with the shape and the head is
+    cleared again (on the current stream)."""
     key = (device, slot)
     ws = _WORKSPACES.get(key)
     if ws is None or ws.numel() < need:
         ws = torch.zeros(max(need, 1 << 20), dtype=torch.uint8, device=device)
         _WORKSPACES[key] = ws
-    elif _WS_SHAPE.get(key) != shape and ticket_bytes > 0:
-        with torch.cuda.device(device):
-            ws[:ticket_bytes].zero_()
-    _WS_SHAPE[key] = shape
+    else:
+        prev_shape, prev_bytes = _WS_SHAPE[key]
+        if prev_shape != shape and max(prev_bytes, ticket_bytes) > cabi.SMLM_TICKET_HEAD:
+            with on_device(ws):
+                ws[:ticket_bytes].zero_()
+    _WS_SHAPE[key] = (shape, ticket_bytes)
     return ws
 
 
@@ -186,7 +226,7 @@ def wgrad_workspace(device, T: int, npart: int, rank: int, h0: int, h1: int = 0,
 def wgrad(g_table, p, q, part_indptr, plan: Plan, transposed: bool, part_scale=None, accumulate=False,
           grad_fp32=False, workspace=None):
     ws = workspace if workspace is not None else wgrad_workspace(p.device, plan.T, plan.nseg, p.size(1), q.size(1))
-    with torch.cuda.device(p.device):
+    with on_device(p):
         check(lib.smlm_b200_wgrad(g_table.data_ptr(), p.data_ptr(), q.data_ptr(), part_indptr.data_ptr(),
                                   _p(part_scale), plan.buf.data_ptr(), ws.data_ptr(), ws.numel(),
                                   int(part_indptr.numel()) - 1, plan.T, int(p.size(1)), int(q.size(1)),
@@ -201,7 +241,7 @@ def wgrad_pair(dA_table, dB_table, dv, x, v, go, part_indptr, plan: Plan, rank: 
     ``fwd``, and in addition the call shares its ``workspace`` with none of those kernels."""
     ws = workspace if workspace is not None else wgrad_workspace(go.device, plan.T, plan.nseg, rank, go.size(1),
                                                                  x.size(1))
-    with torch.cuda.device(go.device):
+    with on_device(go):
         check(lib.smlm_b200_wgrad_pair(dA_table.data_ptr(), dB_table.data_ptr(), dv.data_ptr(), x.data_ptr(),
                                        v.data_ptr(), go.data_ptr(), part_indptr.data_ptr(), _p(part_ids),
                                        _p(part_scale), plan.buf.data_ptr(), ws.data_ptr(), ws.numel(), int(n_table),
@@ -216,7 +256,7 @@ def bwd(dx, dA_table, dB_table, dv, go, x, v, wa_table, wb_table, plan: Plan, ra
     """Backward over the train partitions ``plan.indptr``; rows = go.size(0)."""
     ws = workspace if workspace is not None else wgrad_workspace(go.device, plan.T, plan.nseg, rank, go.size(1),
                                                                  x.size(1))
-    with torch.cuda.device(go.device):
+    with on_device(go):
         check(lib.smlm_b200_bwd(dx.data_ptr(), dA_table.data_ptr(), dB_table.data_ptr(), dv.data_ptr(),
                                 go.data_ptr(), x.data_ptr(), v.data_ptr(), wa_table.data_ptr(),
                                 wb_table.data_ptr(), _p(part_ids), _p(part_scale), plan.indptr.data_ptr(),
@@ -271,7 +311,7 @@ class ProjSet:
 def fwd_multi(ps: ProjSet, plan: Plan, rank: int, is_row_major=False, seg_ids=None, seg_scale=None,
               accumulate=False, independent=False):
     """``fwd`` for every projection of the set in one launch."""
-    with torch.cuda.device(ps.ref.device):
+    with on_device(ps.ref):
         check(lib.smlm_b200_fwd_multi(ps.ptr, ps.n, _p(seg_ids), _p(seg_scale), plan.buf.data_ptr(),
                                       int(ps.keep[0]["wa"].numel()), plan.T, plan.nseg, int(rank), ps._dt("x"),
                                       int(bool(is_row_major)), int(bool(accumulate)), int(bool(independent)),
@@ -281,7 +321,7 @@ def fwd_multi(ps: ProjSet, plan: Plan, rank: int, is_row_major=False, seg_ids=No
 def bwd_dx_multi(ps: ProjSet, plan: Plan, rank: int, is_row_major=False, part_ids=None, part_scale=None,
                  independent=False):
     """``bwd_dx`` for every projection of the set in one launch."""
-    with torch.cuda.device(ps.ref.device):
+    with on_device(ps.ref):
         check(lib.smlm_b200_bwd_dx_multi(ps.ptr, ps.n, _p(part_ids), _p(part_scale), plan.buf.data_ptr(),
                                          int(ps.keep[0]["wa"].numel()), plan.T, plan.nseg, int(rank), ps._dt("go"),
                                          int(bool(is_row_major)), int(bool(independent)), _stream(ps.ref)),
@@ -307,7 +347,7 @@ def wgrad_pair_multi(ps: ProjSet, part_indptr, plan: Plan, rank: int, is_row_maj
     """``wgrad_pair`` for every projection of the set in one launch; ``which`` restricts it to dB (reads v, go)
     or dA (reads dv, x)."""
     ws = workspace if workspace is not None else wgrad_multi_workspace(ps, plan.T, plan.nseg, rank, which=which)
-    with torch.cuda.device(ps.ref.device):
+    with on_device(ps.ref):
         check(lib.smlm_b200_wgrad_select_multi(ps.ptr, ps.n, int(which), part_indptr.data_ptr(), _p(part_ids),
                                                _p(part_scale), plan.buf.data_ptr(), ws.data_ptr(), ws.numel(),
                                                int(n_table), int(part_indptr.numel()) - 1, plan.T, int(rank),
@@ -322,7 +362,7 @@ def wgrad_pair_multi(ps: ProjSet, part_indptr, plan: Plan, rank: int, is_row_maj
 
 def rms_norm(out: torch.Tensor, rms_out: torch.Tensor, x: torch.Tensor, w: torch.Tensor, eps: float):
     """out = x * rsqrt(mean(x^2) + eps) * w per row, rms_out [rows, 1] fp32 gets the rsqrt."""
-    with torch.cuda.device(x.device):
+    with on_device(x):
         check(lib.smlm_b200_rms_norm(out.data_ptr(), rms_out.data_ptr(), x.data_ptr(), w.data_ptr(), int(x.size(0)),
                                      int(x.size(1)), float(eps), _dtype_code(x), _stream(x)), "smlm_b200_rms_norm")
     return out
@@ -334,7 +374,7 @@ def rms_norm_bwd(dx: torch.Tensor, dw: torch.Tensor, go: torch.Tensor, x: torch.
     rows, cols = int(x.size(0)), int(x.size(1))
     need = int(lib.smlm_b200_rms_norm_bwd_workspace_bytes(rows, cols))
     ws = workspace if workspace is not None else torch.empty(max(need, 16), dtype=torch.uint8, device=x.device)
-    with torch.cuda.device(x.device):
+    with on_device(x):
         check(lib.smlm_b200_rms_norm_bwd(dx.data_ptr(), dw.data_ptr(), go.data_ptr(), x.data_ptr(), w.data_ptr(),
                                          rms.data_ptr(), ws.data_ptr(), ws.numel(), rows, cols, _dtype_code(x),
                                          int(dw.dtype == torch.float32), _stream(x)), "smlm_b200_rms_norm_bwd")
