@@ -191,20 +191,21 @@ int launch(Kern kern, dim3 grid, int threads, int cluster_x, int smem_bytes, cud
 
 // ---- fused shrink + expand ----------------------------------------------------
 
-template <typename T, int R16, bool RM>
+template <typename T, int R16, bool RM, bool WIDE = false>
 int launch_fused(const FusedArgs& a, const FusedMapsN& tm, int ctas, bool grouped, cudaStream_t stream) {
   const dim3 grid(ctas, 1, 1);
-  return grouped ? launch(fused_kernel<T, R16, RM, true>, grid, kFusedThreads, a.ksplit, FusedSmem<R16, RM>::kTotal,
-                          stream, a, tm)
-                 : launch(fused_kernel<T, R16, RM, false>, grid, kFusedThreads, a.ksplit,
-                          FusedSmem<R16, RM>::kTotal, stream, a, tm);
+  constexpr int smem = FusedSmem<R16, RM, WIDE>::kTotal;
+  return grouped ? launch(fused_kernel<T, R16, RM, true, WIDE>, grid, kFusedThreads, a.ksplit, smem, stream, a, tm)
+                 : launch(fused_kernel<T, R16, RM, false, WIDE>, grid, kFusedThreads, a.ksplit, smem, stream, a, tm);
 }
 
 template <typename T, bool RM>
-int dispatch_fused_r(const FusedArgs& a, const FusedMapsN& tm, int ctas, bool grouped, cudaStream_t stream) {
+int dispatch_fused_r(const FusedArgs& a, const FusedMapsN& tm, int ctas, bool grouped, bool wide, cudaStream_t stream) {
   const int r16 = (a.R + 15) / 16;
   if (r16 <= 1) return launch_fused<T, 1, RM>(a, tm, ctas, grouped, stream);
-  if (r16 <= 2) return launch_fused<T, 2, RM>(a, tm, ctas, grouped, stream);
+  if (r16 <= 2)
+    return wide ? launch_fused<T, 2, RM, true>(a, tm, ctas, grouped, stream)
+                : launch_fused<T, 2, RM>(a, tm, ctas, grouped, stream);
   if (r16 <= 4) return launch_fused<T, 4, RM>(a, tm, ctas, grouped, stream);
   return launch_fused<T, 8, RM>(a, tm, ctas, grouped, stream);
 }
@@ -283,12 +284,15 @@ int run_fused(const FusedJobDesc* jobs, int njobs, const int32_t* ids, const flo
   const int mp = max_pieces_of(T, nseg);
   const int r16b = (R + 15) / 16;
   const int r16 = r16b > 4 ? 8 : (r16b > 2 ? 4 : r16b);
-  const int kc = 64 * fused_chunks(r16);
+  // the wide form for batches of short segments: kGatherMaxLen rows a segment on average, the length up to which a
+  // grouped plan gathers them (both forms measured where they are described)
+  const bool wide = r16 == 2 && T <= static_cast<long long>(kGatherMaxLen) * nseg;
+  const int kc = 64 * fused_chunks(r16, wide);
   // pieces the plan is expected to hold: its capacity, except that a grouped plan turns the short
   // segments of an adapter into one gather piece, so no more than one piece per adapter comes from them
   const int est_pieces = grouped ? std::min(mp, T / piece_rows_for(T) + std::min(nseg, n_table)) : mp;
-  const double stage_kb = 64.0 * kc * 2 / 1024.0 * 1.28, slab_kb = 64.0 * fused_slab(r16) * 2 / 1024.0;
-  const int slots = kNumSMs * fused_ctas_per_sm(r16);
+  const double stage_kb = 64.0 * kc * 2 / 1024.0 * 1.28, slab_kb = 64.0 * fused_slab(r16, wide) * 2 / 1024.0;
+  const int slots = kNumSMs * fused_ctas_per_sm(r16, wide);
   for (int j0 = 0; j0 < njobs; j0 += kFusedMaxJobs) {
     const int nj = std::min(kFusedMaxJobs, njobs - j0);
     // A piece can be split over the KS CTAs of a cluster; pick the KS that minimises the estimated
@@ -306,7 +310,7 @@ int run_fused(const FusedJobDesc* jobs, int njobs, const int32_t* ids, const flo
       const double load = std::max(1.0, std::min<double>(ctas, slots) / kNumSMs);  // CTAs sharing one SM
       for (int j = 0; j < nj; ++j) {
         const FusedJobDesc& d = jobs[j0 + j];
-        const int ksteps = (d.K1 + kc - 1) / kc, nslabs = (d.N2 + fused_slab(r16) - 1) / fused_slab(r16);
+        const int ksteps = (d.K1 + kc - 1) / kc, nslabs = (d.N2 + fused_slab(r16, wide) - 1) / fused_slab(r16, wide);
         if (k > 1 && ((mode != kFusedExpandOnly && ksteps < k) || (mode != kFusedShrinkOnly && nslabs < k)))
           fits = false;
         const int nk = (ksteps + k - 1) / k, ns = (nslabs + k - 1) / k;
@@ -382,11 +386,11 @@ int run_fused(const FusedJobDesc* jobs, int njobs, const int32_t* ids, const flo
     const int ctas = mp * ks * nj;
     int rc;
     if (dtype == SMLM_F16)
-      rc = row_major ? dispatch_fused_r<__half, true>(a, tm, ctas, g, stream)
-                     : dispatch_fused_r<__half, false>(a, tm, ctas, g, stream);
+      rc = row_major ? dispatch_fused_r<__half, true>(a, tm, ctas, g, wide, stream)
+                     : dispatch_fused_r<__half, false>(a, tm, ctas, g, wide, stream);
     else
-      rc = row_major ? dispatch_fused_r<__nv_bfloat16, true>(a, tm, ctas, g, stream)
-                     : dispatch_fused_r<__nv_bfloat16, false>(a, tm, ctas, g, stream);
+      rc = row_major ? dispatch_fused_r<__nv_bfloat16, true>(a, tm, ctas, g, wide, stream)
+                     : dispatch_fused_r<__nv_bfloat16, false>(a, tm, ctas, g, wide, stream);
     if (rc != SMLM_OK) return rc;
   }
   return SMLM_OK;

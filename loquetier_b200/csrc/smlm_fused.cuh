@@ -62,16 +62,18 @@ constexpr int kFusedConsumers = 8;                           // consumer warps
 constexpr int kFusedThreads = (kFusedConsumers + 1) * 32;    // + one producer warp
 constexpr int kFusedCThreads = kFusedConsumers * 32;
 
-#ifndef SMLM_FUSED_CH
-#define SMLM_FUSED_CH 8
-#endif
-// 64-column chunks of IN per ring stage; high ranks trade width for panel space
-// Rank <= 16 is sized so that two CTAs fit on one SM: an independent successor launch can then
-// move in and read while this launch is still writing.
-constexpr int fused_chunks(int r16) { return r16 >= 8 ? 2 : (r16 == 4 ? 4 : (r16 == 2 ? SMLM_FUSED_CH : 4)); }
+// 64-column chunks of IN per ring stage; high ranks trade width for panel space.
+// Ranks up to 32 are sized so that two CTAs fit on one SM: an independent successor launch can then
+// move in and read while this launch is still writing, and one CTA's set-up and turn from reading to
+// writing pass under the other's copies.  At rank 17..32 there is a second form, `wide`: one CTA per SM with twice
+// the width.  Pieces of a few rows only stream panels, W1 as one copy per rank and step, and there the longer
+// copies count for more.  Measured at rank 32, hidden sizes 4096 and 11008, wide against narrow: one-token segments
+// (1024 of 256 adapters, two projections) 191 against 204 us; a quarter-trained batch of 8192 tokens in long and short
+// segments (seven projections) 485 against 408 us, 128 such tokens 90 against 72 us.
+constexpr int fused_chunks(int r16, bool wide) { return r16 >= 8 ? 2 : (wide ? 8 : 4); }
 constexpr int fused_stages(int) { return 2; }
-constexpr int fused_slab(int r16) { return r16 >= 8 ? 128 : (r16 == 4 ? 256 : (r16 == 2 ? 1024 : 512)); }
-constexpr int fused_ctas_per_sm(int r16) { return r16 == 1 ? 2 : 1; }
+constexpr int fused_slab(int r16, bool wide) { return r16 >= 8 ? 128 : (r16 == 4 ? 256 : (wide ? 1024 : 512)); }
+constexpr int fused_ctas_per_sm(int r16, bool wide) { return r16 <= 2 && !wide ? 2 : 1; }
 
 struct FusedMaps {
   CUtensorMap in8;    // IN boxes of 8 rows x 64 columns (pieces of at most 8 rows)
@@ -80,11 +82,12 @@ struct FusedMaps {
   CUtensorMap out8;   // OUT boxes of 8 rows x 64 columns (last block of a piece of 8k rows)
 };
 
-template <int R16, bool RM>
+template <int R16, bool RM, bool WIDE>
 struct FusedSmem {
+  static_assert(!WIDE || R16 == 2, "only ranks 17..32 have a wide form");
   static constexpr int NT = R16 * 2;            // n-tiles of 8 in the shrink
   static constexpr int KP = R16 * 16;           // padded rank
-  static constexpr int CH = fused_chunks(R16);
+  static constexpr int CH = fused_chunks(R16, WIDE);
   static constexpr int KC = 64 * CH;            // K1 columns per ring stage
   static constexpr int WPad = KC * 2 + 16;      // bytes between W1 rows in shared memory ([R][K1] layout)
   static constexpr int XPad = KC * 2 + 16;      // bytes between the rows of a gather piece in a ring stage
@@ -95,21 +98,26 @@ struct FusedSmem {
   static constexpr int kW1Bytes = (kW1Raw + 1023) / 1024 * 1024;
   static constexpr int kStage = kXBytes + kW1Bytes;
   static constexpr int kRing = kStages * kStage;
-  // phase 3 lives in the space of the ring: two W2 slabs, then per warp two 16 x 128 staging blocks
-  static constexpr int SLAB = fused_slab(R16);
+  // phase 3 lives in the space of the ring: two W2 slabs, then per warp kOutSlots 16 x 64 staging blocks
+  static constexpr int SLAB = fused_slab(R16, WIDE);
   static constexpr int kW2Slab = SLAB * KP * 2;
   static constexpr int kOutOff = 2 * kW2Slab;
-  static constexpr int kStageOut = kFusedConsumers * 2 * 4096;
+  static constexpr int kOutSlots = R16 == 2 && !WIDE ? 2 : 4;  // tensor stores a warp keeps in flight
+  static constexpr int kStageOut = kFusedConsumers * kOutSlots * 2048;
   static constexpr int kPhase3 = kOutOff + kStageOut;
   static constexpr int kUnion = kRing > kPhase3 ? kRing : kPhase3;
-  static constexpr int kRedOff = kUnion;
-  static constexpr int kRed = kFusedConsumers * 16 * KP * 4;   // one 16 x KP fp32 block per consumer warp
-  static constexpr int kMidOff = kRedOff + kRed;
+  // one 16 x KP fp32 block per consumer warp; in the narrow form of rank 17..32 it takes the place of the staging blocks, which
+  // costs a barrier (and an earlier one of the cluster) and makes room for the second CTA
+  static constexpr bool kRedInRing = R16 == 2 && !WIDE;
+  static constexpr int kRed = kFusedConsumers * 16 * KP * 4;
+  static constexpr int kRedOff = kRedInRing ? kOutOff : kUnion;
+  static constexpr int kMidOff = kRedInRing ? kUnion : kRedOff + kRed;
   static constexpr int kMid = kBM * KP * 2;
   static constexpr int kRowOff = kMidOff + kMid;                  // int[kBM]: token rows of a gather piece
   static constexpr int kBarOff = kRowOff + kBM * 4;
   static constexpr int kTotal = kBarOff + 2 * kStages * 8 + 1024;  // + alignment slack
-  static_assert(kTotal <= (fused_ctas_per_sm(R16) == 2 ? 113 : 227) * 1024, "shared memory budget");
+  static_assert(!kRedInRing || kOutOff + kRed <= kUnion, "the partial sums must fit behind the slabs");
+  static_assert(kTotal <= (fused_ctas_per_sm(R16, WIDE) == 2 ? 113 : 227) * 1024, "shared memory budget");
   static_assert(kW2Slab % 1024 == 0 && kStage % 1024 == 0, "swizzled tiles need 1024-byte alignment");
 };
 
@@ -165,11 +173,11 @@ __device__ __forceinline__ void cluster_wait() {
   asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
 }
 
-template <typename T, int R16, bool RM, bool GATHER>
-__global__ void __launch_bounds__(kFusedThreads, fused_ctas_per_sm(R16)) fused_kernel(
+template <typename T, int R16, bool RM, bool GATHER, bool WIDE>
+__global__ void __launch_bounds__(kFusedThreads, fused_ctas_per_sm(R16, WIDE)) fused_kernel(
     const __grid_constant__ FusedArgs a, const __grid_constant__ FusedMapsN tmn) {
   extern __shared__ unsigned char smem_raw[];
-  using SM = FusedSmem<R16, RM>;
+  using SM = FusedSmem<R16, RM, WIDE>;
   constexpr int NT = SM::NT;
   constexpr int KP = SM::KP;
   constexpr int S = SM::kStages;
@@ -400,6 +408,7 @@ __global__ void __launch_bounds__(kFusedThreads, fused_ctas_per_sm(R16)) fused_k
 
   // ======================= phase 2: reduce the K1 slices, build MID =======================
   float* red = reinterpret_cast<float*>(smem + SM::kRedOff);  // [warp][16][KP]
+  if constexpr (SM::kRedInRing) __syncthreads();   // every stage of the ring has been consumed
   if (warp < NW) {
     const int g = lane >> 2, t = lane & 3;
     float* my = red + warp * 16 * KP;
@@ -460,6 +469,9 @@ __global__ void __launch_bounds__(kFusedThreads, fused_ctas_per_sm(R16)) fused_k
   // leaves (and frees its shared memory) while a peer may still be reading it
   if (reduce_cluster) cluster_arrive();
   __syncthreads();  // MID is complete; the ring is free for phase 3
+  if constexpr (SM::kRedInRing) {
+    if (reduce_cluster) cluster_wait();   // phase 3 writes where the peers have been reading
+  }
 
   // ======================= phase 3: expand over this CTA's N2 slice =======================
   const int nslabs = (N2 + SLAB - 1) / SLAB;
@@ -518,8 +530,8 @@ __global__ void __launch_bounds__(kFusedThreads, fused_ctas_per_sm(R16)) fused_k
         ldsm_x4(dst[kk], mids + r * (XC * 16) + (swz<XC>(r, c) << 4));
       }
     };
-    // per warp four staging blocks of 16 x 64 (2 KB): the tensor stores in flight
-    const uint32_t ostage = base + SM::kOutOff + warp * 8192;
+    // per warp kOutSlots staging blocks of 16 x 64 (2 KB): the tensor stores in flight
+    const uint32_t ostage = base + SM::kOutOff + warp * (SM::kOutSlots * 2048);
     T* const obase = static_cast<T*>(jb.out);
     const int accumulate = jb.accumulate;
     int oslot = 0;
@@ -581,7 +593,7 @@ __global__ void __launch_bounds__(kFusedThreads, fused_ctas_per_sm(R16)) fused_k
               o[j][0] *= sc_w; o[j][1] *= sc_w; o[j][2] *= sc_w; o[j][3] *= sc_w;
             }
           }
-          if (lane == 0) bulk_wait_read<3>();  // the staging block about to be reused has been read
+          if (lane == 0) bulk_wait_read<SM::kOutSlots - 1>();  // the staging block about to be reused has been read
           __syncwarp();
           const uint32_t os = ostage + oslot * 2048;
 #pragma unroll
@@ -602,7 +614,7 @@ __global__ void __launch_bounds__(kFusedThreads, fused_ctas_per_sm(R16)) fused_k
               else tma_store_2d(omap, n0 + grp * 64, pc.row0 + rb * 16, os);
               bulk_commit();
             }
-            oslot = (oslot + 1) & 3;
+            oslot = (oslot + 1) & (SM::kOutSlots - 1);
           } else {
             // ragged tail of the piece, or a gather piece: plain 16-byte stores of the rows that exist
             __syncwarp();
@@ -640,7 +652,9 @@ __global__ void __launch_bounds__(kFusedThreads, fused_ctas_per_sm(R16)) fused_k
     if (lane == 0) bulk_wait<0>();  // shared memory must outlive the tensor stores that read it
     __syncwarp();
   }
-  if (reduce_cluster) cluster_wait();
+  if constexpr (!SM::kRedInRing) {
+    if (reduce_cluster) cluster_wait();
+  }
   if (a.independent) pdl_wait();
 }
 
