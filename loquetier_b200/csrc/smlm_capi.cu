@@ -206,7 +206,9 @@ int dispatch_fused_r(const FusedArgs& a, const FusedMapsN& tm, int ctas, bool gr
   if (r16 <= 2)
     return wide ? launch_fused<T, 2, RM, true>(a, tm, ctas, grouped, stream)
                 : launch_fused<T, 2, RM>(a, tm, ctas, grouped, stream);
-  if (r16 <= 4) return launch_fused<T, 4, RM>(a, tm, ctas, grouped, stream);
+  if (r16 <= 4)
+    return wide ? launch_fused<T, 4, RM, true>(a, tm, ctas, grouped, stream)
+                : launch_fused<T, 4, RM>(a, tm, ctas, grouped, stream);
   return launch_fused<T, 8, RM>(a, tm, ctas, grouped, stream);
 }
 
@@ -284,13 +286,16 @@ int run_fused(const FusedJobDesc* jobs, int njobs, const int32_t* ids, const flo
   const int mp = max_pieces_of(T, nseg);
   const int r16b = (R + 15) / 16;
   const int r16 = r16b > 4 ? 8 : (r16b > 2 ? 4 : r16b);
-  // the wide form for batches of short segments: kGatherMaxLen rows a segment on average, the length up to which a
-  // grouped plan gathers them (both forms measured where they are described)
-  const bool wide = r16 == 2 && T <= static_cast<long long>(kGatherMaxLen) * nseg;
-  const int kc = 64 * fused_chunks(r16, wide);
   // pieces the plan is expected to hold: its capacity, except that a grouped plan turns the short
   // segments of an adapter into one gather piece, so no more than one piece per adapter comes from them
   const int est_pieces = grouped ? std::min(mp, T / piece_rows_for(T) + std::min(nseg, n_table)) : mp;
+  // Ranks 17..64: the wide form for batches of short segments - kGatherMaxLen rows a segment on average, the length
+  // up to which a grouped plan gathers them - and, above rank 32, where the launch does not give every SM a CTA (its
+  // steps are short then, and nothing shares the SM); both forms measured where they are described.
+  const bool wide = (r16 == 2 || r16 == 4) &&
+                    (T <= static_cast<long long>(kGatherMaxLen) * nseg ||
+                     (r16 == 4 && static_cast<long long>(est_pieces) * std::min(njobs, kFusedMaxJobs) < kNumSMs));
+  const int kc = 64 * fused_chunks(r16, wide);
   const double stage_kb = 64.0 * kc * 2 / 1024.0 * 1.28, slab_kb = 64.0 * fused_slab(r16, wide) * 2 / 1024.0;
   const int slots = kNumSMs * fused_ctas_per_sm(r16, wide);
   for (int j0 = 0; j0 < njobs; j0 += kFusedMaxJobs) {

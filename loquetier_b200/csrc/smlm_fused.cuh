@@ -63,17 +63,21 @@ constexpr int kFusedThreads = (kFusedConsumers + 1) * 32;    // + one producer w
 constexpr int kFusedCThreads = kFusedConsumers * 32;
 
 // 64-column chunks of IN per ring stage; high ranks trade width for panel space.
-// Ranks up to 32 are sized so that two CTAs fit on one SM: an independent successor launch can then
+// Ranks up to 64 are sized so that two CTAs fit on one SM: an independent successor launch can then
 // move in and read while this launch is still writing, and one CTA's set-up and turn from reading to
-// writing pass under the other's copies.  At rank 17..32 there is a second form, `wide`: one CTA per SM with twice
-// the width.  Pieces of a few rows only stream panels, W1 as one copy per rank and step, and there the longer
-// copies count for more.  Measured at rank 32, hidden sizes 4096 and 11008, wide against narrow: one-token segments
-// (1024 of 256 adapters, two projections) 191 against 204 us; a quarter-trained batch of 8192 tokens in long and short
-// segments (seven projections) 485 against 408 us, 128 such tokens 90 against 72 us.
-constexpr int fused_chunks(int r16, bool wide) { return r16 >= 8 ? 2 : (wide ? 8 : 4); }
+// writing pass under the other's copies.  At rank 17..64 there is a second form, `wide`: one CTA per SM with twice
+// the width of a step.  Pieces of a few rows only stream panels, W1 as one copy per rank and step, and there the
+// longer copies count for more; so they do, above rank 32, in launches that have no second CTA for an SM.  Measured,
+// hidden sizes 4096 and 11008, us, wide against narrow:
+//   1024 one-token segments of 256 adapters, two projections     rank 32  191 / 204
+//   zipf lengths, seven projections, a quarter trained:
+//     8192 tokens     rank 32  485 / 408    rank 40  845 / 682    rank 64  1031 / 884
+//     1000 tokens     rank 32  102 / 92     rank 40  157 / 142    rank 64  184 / 171
+//     128 tokens      rank 32  90 / 72      rank 40  72 / 87      rank 64  77 / 102
+constexpr int fused_chunks(int r16, bool wide) { return r16 >= 8 ? 2 : (r16 == 4 ? (wide ? 4 : 2) : (wide ? 8 : 4)); }
 constexpr int fused_stages(int) { return 2; }
 constexpr int fused_slab(int r16, bool wide) { return r16 >= 8 ? 128 : (r16 == 4 ? 256 : (wide ? 1024 : 512)); }
-constexpr int fused_ctas_per_sm(int r16, bool wide) { return r16 <= 2 && !wide ? 2 : 1; }
+constexpr int fused_ctas_per_sm(int r16, bool wide) { return r16 <= 4 && !wide ? 2 : 1; }
 
 struct FusedMaps {
   CUtensorMap in8;    // IN boxes of 8 rows x 64 columns (pieces of at most 8 rows)
@@ -84,7 +88,7 @@ struct FusedMaps {
 
 template <int R16, bool RM, bool WIDE>
 struct FusedSmem {
-  static_assert(!WIDE || R16 == 2, "only ranks 17..32 have a wide form");
+  static_assert(!WIDE || R16 == 2 || R16 == 4, "only ranks 17..64 have a wide form");
   static constexpr int NT = R16 * 2;            // n-tiles of 8 in the shrink
   static constexpr int KP = R16 * 16;           // padded rank
   static constexpr int CH = fused_chunks(R16, WIDE);
@@ -98,17 +102,17 @@ struct FusedSmem {
   static constexpr int kW1Bytes = (kW1Raw + 1023) / 1024 * 1024;
   static constexpr int kStage = kXBytes + kW1Bytes;
   static constexpr int kRing = kStages * kStage;
+  static constexpr bool kRedInRing = (R16 == 2 || R16 == 4) && !WIDE;
   // phase 3 lives in the space of the ring: two W2 slabs, then per warp kOutSlots 16 x 64 staging blocks
   static constexpr int SLAB = fused_slab(R16, WIDE);
   static constexpr int kW2Slab = SLAB * KP * 2;
   static constexpr int kOutOff = 2 * kW2Slab;
-  static constexpr int kOutSlots = R16 == 2 && !WIDE ? 2 : 4;  // tensor stores a warp keeps in flight
+  static constexpr int kOutSlots = kRedInRing ? 2 : 4;         // tensor stores a warp keeps in flight
   static constexpr int kStageOut = kFusedConsumers * kOutSlots * 2048;
   static constexpr int kPhase3 = kOutOff + kStageOut;
   static constexpr int kUnion = kRing > kPhase3 ? kRing : kPhase3;
-  // one 16 x KP fp32 block per consumer warp; in the narrow form of rank 17..32 it takes the place of the staging blocks, which
+  // one 16 x KP fp32 block per consumer warp; in the narrow form of rank 17..64 it takes the place of the staging blocks, which
   // costs a barrier (and an earlier one of the cluster) and makes room for the second CTA
-  static constexpr bool kRedInRing = R16 == 2 && !WIDE;
   static constexpr int kRed = kFusedConsumers * 16 * KP * 4;
   static constexpr int kRedOff = kRedInRing ? kOutOff : kUnion;
   static constexpr int kMidOff = kRedInRing ? kUnion : kRedOff + kRed;

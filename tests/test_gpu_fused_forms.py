@@ -1,4 +1,4 @@
-"""The two forms of the fused kernel at ranks above 16: batches on either side of the rule (rows per segment) and at
+"""The two forms of the fused kernel at ranks 17 to 64: batches on either side of the rule (rows per segment) and at
 it, alone, grouped, and split over clusters, against the oracle.  Tolerance: v and y are rounded to 16 bits (2^-9
 relative in bf16) after fp32 sums, and y carries v's rounding: rtol = atol = 1e-2 as for the other forward tests."""
 import pytest
@@ -10,9 +10,9 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
-@pytest.mark.parametrize("rank", [24, 32])
+@pytest.mark.parametrize("rank", [24, 32, 40, 64])
 @pytest.mark.parametrize("rm", [False, True])
-@pytest.mark.parametrize("lens", [[1] * 9, [8] * 6, [8] * 5 + [9], [64, 65, 1, 17, 130], [0, 3, 0, 0, 5]])
+@pytest.mark.parametrize("lens", [[1] * 9, [8] * 6, [8] * 5 + [9], [64, 65, 1, 17, 130], [0, 3, 0, 0, 5], [9] * 150])
 @pytest.mark.parametrize("split", [0, 1, 2, 4])
 def test_forms_on_either_side_of_the_rule(dtype, rank, rm, lens, split):
     from gpu_util import check_forward
