@@ -595,13 +595,14 @@ inline RmsShape rms_shape(int n8) {
   if (n8 <= 2048) return {1024, 2};
   return {1024, 0};
 }
-// persistent CTAs: about 2048 threads per SM in the forward, 512 in the backward (which holds two rows
-// of x, two of gO and its share of dW in registers)
+// persistent CTAs: about 2048 threads per SM in the forward; the backward holds two rows of x, two of gO and its
+// share of dW in registers
 inline int rms_fwd_grid(int rows, int cols) {
   return std::max(1, std::min(rows, kNumSMs * (2048 / rms_shape(cols / 8).threads)));
 }
 inline int rms_bwd_grid(int rows, int cols) {
-  return std::max(1, std::min(rows, kNumSMs * std::max(1, 512 / rms_shape(cols / 8).threads)));
+  const RmsShape sh = rms_shape(cols / 8);
+  return std::max(1, std::min(rows, kNumSMs * rms_bwd_ctas_per_sm(sh.vpt, sh.threads)));
 }
 
 template <typename T, int VPT, int NT>
