@@ -35,9 +35,9 @@ extern "C" {
 /* Bytes of the workspace of smlm_b200_batch_decode for this batch shape.  The reference asks its
  * caller for a fixed 64 MiB `tmpbuf` (loquetier_ops.cc:152-153); here the size follows the batch.  The
  * head of the workspace - smlm_b200_batch_decode_ticket_bytes(...) bytes - must be zero when a launch starts;
- * every launch leaves it zeroed again.  So: zero-fill once after allocation, and zero the head again whenever
- * batch_size * num_kv_heads differs from the previous call's on the same workspace (a different shape moves the
- * boundary between the tickets and the parked softmax states).  Launches that may overlap in time must not share
+ * every launch leaves it zeroed again.  So: zero-fill once after allocation, and zero the head again whenever its
+ * size differs from the previous call's on the same workspace (the boundary between the tickets and the parked softmax
+ * states has moved; the head is the same for all batches of up to 16384 batch_size * num_kv_heads).  Launches that may overlap in time must not share
  * a workspace. */
 size_t smlm_b200_batch_decode_workspace_bytes(int batch_size, int num_qo_heads, int num_kv_heads);
 size_t smlm_b200_batch_decode_ticket_bytes(int batch_size, int num_kv_heads);
