@@ -17,8 +17,8 @@
 // number of query heads that share the kv head - they are the columns of one tensor-core tile.  Long
 // sequences of small batches are cut into up to `splits` ranges of key tiles so that the machine is filled; the
 // partial softmax states go through a workspace and the CTA that finishes last (a ticket, no waiting)
-// merges them in range order - a fixed order, so the result does not depend on scheduling.  In batches that
-// need no ranges the longest requests go first, so that the launch ends on its shortest CTAs.
+// merges them in range order - a fixed order, so the result does not depend on scheduling.  In batches of long
+// requests that need no ranges the longest go first, so that the launch ends on its shortest CTAs.
 #pragma once
 #include "smlm_common.cuh"
 
@@ -138,7 +138,7 @@ constexpr int kPdQOff = kPdWarps * kPdWarpRing;      // rotated queries [8 rows]
 constexpr int kPdRotOff = kPdQOff + 8 * kPdDim * 2;  // frequency pairs: step of a warp, step of 8 keys, frequencies
 constexpr int kPdSmem = kPdRotOff + 2 * 512 + 256;
 constexpr int kPdStep = kPdWarps * kPdTile;          // keys between two tiles of a warp
-constexpr int kPdMaxSorted = 512;                    // requests whose ranks a CTA finds for itself
+constexpr int kPdMaxSorted = 128;                    // requests whose ranks a CTA finds for itself
 constexpr int kPdReseed = 16;                        // tiles after which the rotation is computed afresh
 constexpr float kPdRaise = 8.0f;                     // a head's maximum is raised when exceeded by this much (log2)
 

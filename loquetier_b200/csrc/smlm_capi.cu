@@ -663,6 +663,16 @@ inline int decode_min_tiles(int total_pages, int page_size, int num_kv_heads) {
   return static_cast<int>(std::max<long long>(kPdWarps, std::min<long long>(32, tiles / (3 * kNumSMs))));
 }
 
+// Whether a batch without ranges takes its longest requests first.  Every CTA ranks the requests for itself, about 2 us
+// at 128 of them and growing with the square, so it pays where CTAs are long and the launch has a tail: more CTAs than
+// are resident, at most 128 requests, 96 tiles (1536 keys) each on average.  Unsorted against sorted, append + decode:
+// 128 requests of 512..4096 keys 218 / 189 us, 64 of 200..4000 116 / 107, 120 of 2000..2400 128 / 127; but 57 of 1000
+// 61 / 64, 200 of 100..1400 116 / 127, 256 of 20..200 40 / 72.
+inline bool decode_sorted(int batch, int num_kv_heads, int total_pages, int page_size) {
+  const long long tiles = static_cast<long long>(total_pages) * page_size / kPdTile;
+  return batch <= kPdMaxSorted && static_cast<long long>(batch) * num_kv_heads > 3 * kNumSMs && tiles >= 96LL * batch;
+}
+
 inline size_t decode_ticket_bytes(int batch, int num_kv_heads) {
   return ticket_head(static_cast<size_t>(batch) * num_kv_heads * sizeof(int));
 }
@@ -1222,8 +1232,7 @@ int smlm_b200_batch_decode(void* o, const void* q, const void* const* kv_ptrs, c
   a.batch = batch_size; a.num_kv_heads = num_kv_heads; a.num_layers = num_layers; a.layer_idx = layer_idx;
   a.page_size = page_size; a.total_pages = total_pages;
   a.min_tiles = decode_min_tiles(total_pages, page_size, num_kv_heads);
-  // longest requests first where the CTAs take more than one round and the ranks are cheap to find
-  a.sorted = a.splits == 1 && batch_size <= kPdMaxSorted && batch_size * num_kv_heads > 3 * kNumSMs ? 1 : 0;
+  a.sorted = a.splits == 1 && decode_sorted(batch_size, num_kv_heads, total_pages, page_size) ? 1 : 0;
   a.log2_theta = std::log2(rope_theta);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   return dtype == SMLM_F16 ? dispatch_decode<__half>(a, group, st) : dispatch_decode<__nv_bfloat16>(a, group, st);

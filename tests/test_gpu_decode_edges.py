@@ -23,22 +23,25 @@ def _cache(seed, seqlens, N, P, dtype):
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
-@pytest.mark.parametrize("group,batch", [(1, 3), (4, 3), (8, 2), (4, 60), (2, 65), (8, 57)])
+@pytest.mark.parametrize("group,batch", [(1, 3), (4, 3), (8, 2), (4, 60), (2, 65), (8, 57), (1, 127), (1, 128), (1, 129)])
 def test_decode_at_the_edges_of_tiles_ranges_and_ranks(dtype, group, batch):
     """Tiles of 16 keys, a warp's step of 64, the rotation computed afresh every 1024 keys; small batches are cut into
-    ranges, from 56 requests of 8 heads on the requests go by length: equal lengths, empty requests and a last
-    request among them, batches that are no multiple of four."""
+    ranges.  From 56 requests of 8 heads to 128 the requests go by length if the page table holds 96 tiles for each -
+    entries no request uses count - with equal lengths, empty requests and batches that are no multiple of four among
+    them; the order must not show."""
     from loquetier_b200 import kvcache
     N, P = 8, 16
     edge = [1023, 1024, 1025, 2100, 15, 16, 17, 63, 64, 65, 0, 1, 128, 129, 64, 0, 17]
-    seqlens = (edge * 4)[:batch] if batch > 3 else [1025, 2100, 17][:batch]
+    seqlens = (edge * 4 + [3, 20] * 40)[:batch] if batch > 3 else [1025, 2100, 17][:batch]
     host, d = _cache(50 + group + batch, seqlens, N, P, dtype)
     q = torch.randn((batch, N * group, 128), generator=torch.Generator().manual_seed(batch)).to(dtype)
+    ptrs = d["ptrs"]
+    padded = torch.cat([ptrs, ptrs[:1].expand(max(0, 97 * batch - ptrs.numel()))]).contiguous()
     outs = []
-    for _ in range(2):
+    for table in ((ptrs, ptrs) if batch <= 3 else (ptrs, padded)):
         o = torch.full(q.shape, float("nan"), dtype=dtype, device=DEV)
         word = torch.zeros(1, dtype=torch.int32, device=DEV)
-        kvcache.batch_decode_into(o, q.to(DEV), d["ptrs"], d["ind"], d["last"], 1, 0, N, THETA, P, status_word=word)
+        kvcache.batch_decode_into(o, q.to(DEV), table, d["ind"], d["last"], 1, 0, N, THETA, P, status_word=word)
         assert int(word.item()) == 0
         outs.append(o)
     assert torch.equal(outs[0], outs[1])   # merged in a fixed order
