@@ -60,3 +60,41 @@ def test_decode_scores_that_grow_along_the_sequence():
     o = torch.empty(q.shape, dtype=q.dtype, device=DEV)
     kvcache.batch_decode_into(o, q.to(DEV), d["ptrs"], d["ind"], d["last"], 1, 0, N, THETA, P)
     assert_close(o, A.batch_decode(q, pages, indptr, last, 0, THETA), what="raised maxima")
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("group,batch", [(4, 60), (8, 57), (1, 130)])
+def test_decode_weight_of_a_key_that_dominates_late_is_not_rounded(dtype, group, batch):
+    """Softmax weights are rounded to 16 bits relative to the largest score met so far, so the key that sets it has the
+    weight one exactly, in whatever tile it comes.  One key in the second tile of its warp dominates, by 1 to 7.9 in the
+    base-2 score; its value is the only one that is not zero.  Query and key lie in a dimension that this rope base does
+    not turn and their product is exact, so the result is known in float64 and is off by its own rounding only: half a
+    unit of the storage type (and 2^-18 relative for the fp32 exponential, sums and reciprocal)."""
+    from loquetier_b200 import kvcache
+    N, P, L, at, dim = 8, 16, 192, 69, 63
+    bits, k = (8, 16.0) if dtype == torch.bfloat16 else (11, 16.0)
+    qscale = 1.4426950408889634 / 128 ** 0.5
+    g = torch.Generator().manual_seed(group)
+    cand = (torch.rand(20000, generator=g, dtype=torch.float64) * 6.9 + 1.0).div(k * qscale).to(dtype).double()
+    scaled = cand * qscale
+    cand = cand[((scaled * (1 + 1e-5)).to(dtype) == (scaled * (1 - 1e-5)).to(dtype))]   # its rounding is beyond doubt
+    q1 = cand[torch.randperm(cand.numel(), generator=g)[:batch * N * group]].view(batch, N * group)
+    q = torch.zeros((batch, N * group, 128), dtype=dtype)
+    q[:, :, dim] = q1.to(dtype)
+    npg = L // P
+    pages = torch.zeros((batch * npg, 1, 2, N, P, 128), dtype=dtype)
+    v = torch.randn((batch, N, 128), generator=g).to(dtype)
+    for b in range(batch):
+        pg = pages[b * npg + at // P, 0]
+        pg[0, :, at % P, dim] = k
+        pg[1, :, at % P] = v[b]
+    pd = pages.to(DEV)
+    ptrs = torch.tensor([p.data_ptr() for p in pd], dtype=torch.int64, device=DEV)
+    ind = torch.arange(0, (batch + 1) * npg, npg, dtype=torch.int32, device=DEV)
+    last = torch.full((batch,), P, dtype=torch.int32, device=DEV)
+    o = torch.empty(q.shape, dtype=dtype, device=DEV)
+    kvcache.batch_decode_into(o, q.to(DEV), ptrs, ind, last, 1, 0, N, 1e30, P)
+    w = torch.exp2((q1 * qscale).to(dtype).double() * k)
+    want = (w / (w + (L - 1))).unsqueeze(-1) * v.double().repeat_interleave(group, dim=1)
+    half = torch.exp2(torch.floor(torch.log2(want.abs().clamp_min(2.0 ** -14))) - bits)   # half a unit in the last place
+    assert ((o.cpu().double() - want).abs() <= half * 1.0001 + want.abs() * 2.0 ** -18).all()
