@@ -501,7 +501,7 @@ __global__ void __launch_bounds__(kPdWarps * 32, 3) paged_decode_kernel(const Pd
       }
     }
     if (ranges == 1) {
-      O[h * kPdDim] = static_cast<T>(l > 0.f ? acc * (1.0f / l) : 0.f);   // a request without keys gives zeros
+      O[h * kPdDim] = static_cast<T>(l == 0.f ? 0.f : acc * (1.0f / l));   // no keys: zeros; a NaN stays one
     } else {
       float* r = part + (static_cast<size_t>(h) * S + s) * REC;
       if (tid == 0) {
@@ -549,7 +549,7 @@ __global__ void __launch_bounds__(kPdWarps * 32, 3) paged_decode_kernel(const Pd
         acc += oz[z] * wt;
       }
     }
-    O[h * kPdDim] = static_cast<T>(l > 0.f ? acc * (1.0f / l) : 0.f);
+    O[h * kPdDim] = static_cast<T>(l == 0.f ? 0.f : acc * (1.0f / l));
   }
 }
 

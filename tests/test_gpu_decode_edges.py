@@ -98,3 +98,29 @@ def test_decode_weight_of_a_key_that_dominates_late_is_not_rounded(dtype, group,
     want = (w / (w + (L - 1))).unsqueeze(-1) * v.double().repeat_interleave(group, dim=1)
     half = torch.exp2(torch.floor(torch.log2(want.abs().clamp_min(2.0 ** -14))) - bits)   # half a unit in the last place
     assert ((o.cpu().double() - want).abs() <= half * 1.0001 + want.abs() * 2.0 ** -18).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("batch", [4, 60])   # cut into ranges, and not
+def test_decode_not_a_number_shows_in_the_heads_it_enters(dtype, batch):
+    """A NaN or an infinity in one query head or one key makes the heads that see it NaN - never zeros, which would pass
+    for a result - and leaves all others as they are."""
+    from loquetier_b200 import kvcache
+    N, group, P, L = 8, 4, 16, 600
+    _, d = _cache(90 + batch, [L] * batch, N, P, dtype)
+    q = torch.randn((batch, N * group, 128), generator=torch.Generator().manual_seed(91)).to(dtype)
+    run = lambda: kvcache.batch_decode_into(torch.empty(q.shape, dtype=dtype, device=DEV), q.to(DEV), d["ptrs"], d["ind"],
+                                            d["last"], 1, 0, N, THETA, P)
+    clean = run()
+    assert torch.isfinite(clean.float()).all()
+    bad = torch.zeros(q.shape[:2], dtype=torch.bool, device=DEV)
+    q[1, 5, 17] = float("nan")                                     # one query head
+    bad[1, 5] = True
+    npg = -(-L // P)
+    d["keep"][2 * npg + 300 // P][0, 0, 3, 300 % P, 9] = float("nan")   # one key of request 2, kv head 3
+    bad[2, 3 * group:4 * group] = True
+    d["keep"][3 * npg][0, 0, 6, :, 40] = float("inf")              # a whole tile of keys of request 3, kv head 6
+    bad[3, 6 * group:7 * group] = True
+    o = run()
+    assert torch.isnan(o[bad].float()).all()
+    assert torch.equal(o[~bad], clean[~bad])
