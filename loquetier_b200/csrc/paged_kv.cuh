@@ -39,7 +39,6 @@ struct PdArgs {
   int* tickets;                   // [B * Nkv], zero between launches
   float* partial;                 // [B * Nq * splits * kPdRec]
   int batch, num_kv_heads, num_layers, layer_idx, page_size, splits, total_pages;
-  int min_tiles;                  // a range is not made shorter than this many tiles
   int sorted;                     // 1: CTAs take the requests in descending order of their length (batch <= kPdMaxSorted)
   float log2_theta;               // log2(rope base)
 };
@@ -228,7 +227,11 @@ __global__ void __launch_bounds__(kPdWarps * 32, 3) paged_decode_kernel(const Pd
   }
   const int seq_len = npages > 0 ? (npages - 1) * P + last_valid : 0;
   const int ntiles = (seq_len + kPdTile - 1) / kPdTile;
-  const int per = max((ntiles + S - 1) / S, a.min_tiles);
+  // The ranges follow from the request's own length, whatever else the batch or its page table holds.  Longer ranges for
+  // the shorter requests of an uneven batch (a share of the machine each) were up to 17 % faster (20 requests of 100..4000
+  // keys and 4 kv heads, 24 against 29 us) but rounded more weights: every warp's largest is exact, and with fewer ranges
+  // there are fewer of them (error against 64 bits up to 1 % larger).
+  const int per = max((ntiles + S - 1) / S, kPdWarps);        // a tile per warp at least
   const int ranges = max(1, (ntiles + per - 1) / per);        // ranges this request is cut into
   if (s >= ranges) return;
   const int tile0 = s * per;

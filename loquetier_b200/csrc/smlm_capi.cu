@@ -656,13 +656,6 @@ inline int decode_splits(int batch, int num_kv_heads) {
   return std::max(1, std::min(kPdMaxSplits, (3 * kNumSMs + ctas - 1) / ctas));
 }
 
-// The shortest range worth a CTA: what an even share of the batch's tiles (the pages bound them from above) would
-// be, but no more than 32 tiles (8 per warp cover a CTA's set-up) and a tile per warp at least.
-inline int decode_min_tiles(int total_pages, int page_size, int num_kv_heads) {
-  const long long tiles = static_cast<long long>(total_pages) * page_size / kPdTile * num_kv_heads;
-  return static_cast<int>(std::max<long long>(kPdWarps, std::min<long long>(32, tiles / (3 * kNumSMs))));
-}
-
 // Whether a batch without ranges takes its longest requests first.  Every CTA ranks the requests for itself, about 2 us
 // at 128 of them and growing with the square, so it pays where CTAs are long and the launch has a tail: more CTAs than
 // are resident, at most 128 requests, 96 tiles (1536 keys) each on average.  Unsorted against sorted, append + decode:
@@ -1231,7 +1224,6 @@ int smlm_b200_batch_decode(void* o, const void* q, const void* const* kv_ptrs, c
                                                               decode_ticket_bytes(batch_size, num_kv_heads));
   a.batch = batch_size; a.num_kv_heads = num_kv_heads; a.num_layers = num_layers; a.layer_idx = layer_idx;
   a.page_size = page_size; a.total_pages = total_pages;
-  a.min_tiles = decode_min_tiles(total_pages, page_size, num_kv_heads);
   a.sorted = a.splits == 1 && decode_sorted(batch_size, num_kv_heads, total_pages, page_size) ? 1 : 0;
   a.log2_theta = std::log2(rope_theta);
   cudaStream_t st = static_cast<cudaStream_t>(stream);

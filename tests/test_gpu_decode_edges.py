@@ -124,3 +124,32 @@ def test_decode_not_a_number_shows_in_the_heads_it_enters(dtype, batch):
     o = run()
     assert torch.isnan(o[bad].float()).all()
     assert torch.equal(o[~bad], clean[~bad])
+
+
+@pytest.mark.parametrize("spare", [0, 1, 3000])
+def test_decode_ranges_follow_the_requests_and_not_the_page_table(spare):
+    """A page table may be longer than the pages in use (a captured step keeps its arguments).  The ranges a request is
+    cut into are seen from the states parked in the workspace: as many as its length asks for, with any table."""
+    from loquetier_b200 import kvcache
+    from loquetier_b200.cabi import lib
+    N, group, P, REC = 8, 4, 16, 132
+    seqlens = [1024, 2000, 40, 600]
+    host, d = _cache(61, seqlens, N, P, torch.bfloat16)
+    batch = len(seqlens)
+    q = torch.randn((batch, N * group, 128), generator=torch.Generator().manual_seed(62)).to(torch.bfloat16)
+    head = lib.smlm_b200_batch_decode_ticket_bytes(batch, N)
+    ws = torch.zeros(lib.smlm_b200_batch_decode_workspace_bytes(batch, N * group, N), dtype=torch.uint8, device=DEV)
+    ws[head:].view(torch.float32).fill_(float("nan"))
+    table = torch.cat([d["ptrs"], d["ptrs"][:1].expand(spare)]).contiguous()
+    o = torch.empty(q.shape, dtype=q.dtype, device=DEV)
+    kvcache.batch_decode_into(o, q.to(DEV), table, d["ind"], d["last"], 1, 0, N, THETA, P, workspace=ws)
+    parked = ~torch.isnan(ws[head:].view(torch.float32).view(batch, N * group, -1, REC)[..., 0])
+    splits = parked.shape[2]
+    assert splits == min(16, -(-3 * 148 // (batch * N)))
+    for b, n in enumerate(seqlens):
+        tiles = -(-n // 16)
+        per = max(4, -(-tiles // splits))
+        want = -(-tiles // per)
+        want = 0 if want == 1 else want   # one range is not parked
+        assert (parked[b].sum(-1) == want).all(), (n, want)
+    assert_close(o, A.batch_decode(q, *host, 0, THETA), what="long table")
