@@ -39,7 +39,7 @@ struct PdArgs {
   int* tickets;                   // [B * Nkv], zero between launches
   float* partial;                 // [B * Nq * splits * kPdRec]
   int batch, num_kv_heads, num_layers, layer_idx, page_size, splits, total_pages;
-  int sorted;                     // 1: CTAs take the requests in descending order of their length (batch <= kPdMaxSorted)
+  int sort_pages;                 // pages in use from which on the longest requests may go first; negative: never
   float log2_theta;               // log2(rope base)
 };
 
@@ -137,7 +137,7 @@ constexpr int kPdQOff = kPdWarps * kPdWarpRing;      // rotated queries [8 rows]
 constexpr int kPdRotOff = kPdQOff + 8 * kPdDim * 2;  // frequency pairs: step of a warp, step of 8 keys, frequencies
 constexpr int kPdSmem = kPdRotOff + 2 * 512 + 256;
 constexpr int kPdStep = kPdWarps * kPdTile;          // keys between two tiles of a warp
-constexpr int kPdMaxSorted = 128;                    // requests whose ranks a CTA finds for itself
+constexpr int kPdMaxSorted = 192;                    // requests whose ranks a CTA finds for itself
 constexpr int kPdReseed = 16;                        // tiles after which the rotation is computed afresh
 
 // 8 x 8 transpose of 16-bit elements over a warp
@@ -192,25 +192,33 @@ __global__ void __launch_bounds__(kPdWarps * 32, 3) paged_decode_kernel(const Pd
   const int head0 = kvh * G;
 
   pdl_wait();
-  if (a.sorted) {
+  if (a.sort_pages >= 0) {
     // the request whose number of pages has rank b: every CTA counts for itself (whatever the table holds, the
     // ranks are a permutation of the requests)
     int* len = reinterpret_cast<int*>(pd_smem);
     const int n4 = (a.batch + 3) & ~3;
-    for (int i = tid; i < n4; i += kPdWarps * 32) len[i] = i < a.batch ? a.kv_indptr[i + 1] - a.kv_indptr[i] : INT32_MIN;
-    __syncthreads();
-    for (int i = tid; i < a.batch; i += kPdWarps * 32) {
-      const int mine = len[i];
-      int rank = 0;
-      for (int k = 0; k < n4; k += 4) {   // (entries past the batch are never ahead: smallest, and behind)
-        const int4 v = *reinterpret_cast<const int4*>(len + k);
-        rank += (v.x > mine || (v.x == mine && k < i)) + (v.y > mine || (v.y == mine && k + 1 < i)) +
-                (v.z > mine || (v.z == mine && k + 2 < i)) + (v.w > mine || (v.w == mine && k + 3 < i));
-      }
-      if (rank == b) s_last = i;
+    // what the requests hold counts; the table may be longer (a captured step keeps its arguments)
+    const int used = max(0, min(a.kv_indptr[a.batch] - a.kv_indptr[0], a.total_pages));
+    int uneven = 0;   // long requests, and one of them holds more than 5/4 of the mean
+    for (int i = tid; i < n4; i += kPdWarps * 32) {
+      const int n = i < a.batch ? a.kv_indptr[i + 1] - a.kv_indptr[i] : INT32_MIN;
+      len[i] = n;
+      uneven |= used >= a.sort_pages && 4LL * n * a.batch > 5LL * used;
     }
-    __syncthreads();
-    b = s_last;
+    if (__syncthreads_or(uneven)) {
+      for (int i = tid; i < a.batch; i += kPdWarps * 32) {
+        const int mine = len[i];
+        int rank = 0;
+        for (int k = 0; k < n4; k += 4) {   // (entries past the batch are never ahead: smallest, and behind)
+          const int4 v = *reinterpret_cast<const int4*>(len + k);
+          rank += (v.x > mine || (v.x == mine && k < i)) + (v.y > mine || (v.y == mine && k + 1 < i)) +
+                  (v.z > mine || (v.z == mine && k + 2 < i)) + (v.w > mine || (v.w == mine && k + 3 < i));
+        }
+        if (rank == b) s_last = i;
+      }
+      __syncthreads();
+      b = s_last;
+    }
     __syncthreads();   // the ranks' space is the ring's, s_last serves the ranges later
   }
   const int bh = b * a.num_kv_heads + kvh;

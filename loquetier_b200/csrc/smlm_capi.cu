@@ -656,14 +656,19 @@ inline int decode_splits(int batch, int num_kv_heads) {
   return std::max(1, std::min(kPdMaxSplits, (3 * kNumSMs + ctas - 1) / ctas));
 }
 
-// Whether a batch without ranges takes its longest requests first.  Every CTA ranks the requests for itself, about 2 us
-// at 128 of them and growing with the square, so it pays where CTAs are long and the launch has a tail: more CTAs than
-// are resident, at most 128 requests, 96 tiles (1536 keys) each on average.  Unsorted against sorted, append + decode:
-// 128 requests of 512..4096 keys 218 / 189 us, 64 of 200..4000 116 / 107, 120 of 2000..2400 128 / 127; but 57 of 1000
-// 61 / 64, 200 of 100..1400 116 / 127, 256 of 20..200 40 / 72.
-inline bool decode_sorted(int batch, int num_kv_heads, int total_pages, int page_size) {
-  const long long tiles = static_cast<long long>(total_pages) * page_size / kPdTile;
-  return batch <= kPdMaxSorted && static_cast<long long>(batch) * num_kv_heads > 3 * kNumSMs && tiles >= 96LL * batch;
+// Pages in use from which on a batch without ranges takes its longest requests first, unless they are all about equal
+// (the kernel looks); negative: never.  Every CTA ranks the requests for itself, a cost that grows with the square of
+// their number and with the rounds of CTAs, so it pays where CTAs are long and the launch has a tail: more CTAs than are
+// resident, 96 tiles (1536 keys) each on average, up to 192 requests.  Decode alone, 8 kv heads, us, in batch order /
+// longest first, by requests:
+//   512..4096 keys     96  176 / 127    128  212 / 183    160  251 / 223    192  298 / 282    224  338 / 328    256  375 / 376
+//   1540..3000 keys    96  159 / 137    128  201 / 196    160  235 / 223    192  277 / 287    224  317 / 338    256  357 / 376
+//   1600..1700 keys    96  107 / 109    128  149 / 151    160  164 / 174    192  205 / 219   (about equal: left in order)
+// with 4 kv heads the gain lasts to 256 requests (512..4096 keys: 160  150 / 119, 192  175 / 145, 256  213 / 205).
+inline int decode_sort_pages(int batch, int num_kv_heads, int total_pages, int page_size) {
+  if (batch > kPdMaxSorted || static_cast<long long>(batch) * num_kv_heads <= 3 * kNumSMs) return -1;
+  const int pages = (96 * kPdTile * batch + page_size - 1) / page_size;
+  return total_pages >= pages ? pages : -1;   // the requests hold no more than the table does
 }
 
 inline size_t decode_ticket_bytes(int batch, int num_kv_heads) {
@@ -1224,7 +1229,7 @@ int smlm_b200_batch_decode(void* o, const void* q, const void* const* kv_ptrs, c
                                                               decode_ticket_bytes(batch_size, num_kv_heads));
   a.batch = batch_size; a.num_kv_heads = num_kv_heads; a.num_layers = num_layers; a.layer_idx = layer_idx;
   a.page_size = page_size; a.total_pages = total_pages;
-  a.sorted = a.splits == 1 && decode_sorted(batch_size, num_kv_heads, total_pages, page_size) ? 1 : 0;
+  a.sort_pages = a.splits == 1 ? decode_sort_pages(batch_size, num_kv_heads, total_pages, page_size) : -1;
   a.log2_theta = std::log2(rope_theta);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   return dtype == SMLM_F16 ? dispatch_decode<__half>(a, group, st) : dispatch_decode<__nv_bfloat16>(a, group, st);

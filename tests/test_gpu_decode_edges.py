@@ -26,9 +26,8 @@ def _cache(seed, seqlens, N, P, dtype):
 @pytest.mark.parametrize("group,batch", [(1, 3), (4, 3), (8, 2), (4, 60), (2, 65), (8, 57), (1, 127), (1, 128), (1, 129)])
 def test_decode_at_the_edges_of_tiles_ranges_and_ranks(dtype, group, batch):
     """Tiles of 16 keys, a warp's step of 64, the rotation computed afresh every 1024 keys; small batches are cut into
-    ranges.  From 56 requests of 8 heads to 128 the requests go by length if the page table holds 96 tiles for each -
-    entries no request uses count - with equal lengths, empty requests and batches that are no multiple of four among
-    them; the order must not show."""
+    ranges.  Equal lengths, empty requests and batches that are no multiple of four are among them, and a page table with
+    entries that no request uses."""
     from loquetier_b200 import kvcache
     N, P = 8, 16
     edge = [1023, 1024, 1025, 2100, 15, 16, 17, 63, 64, 65, 0, 1, 128, 129, 64, 0, 17]
@@ -153,3 +152,43 @@ def test_decode_ranges_follow_the_requests_and_not_the_page_table(spare):
         want = 0 if want == 1 else want   # one range is not parked
         assert (parked[b].sum(-1) == want).all(), (n, want)
     assert_close(o, A.batch_decode(q, *host, 0, THETA), what="long table")
+
+
+@pytest.mark.parametrize("batch", [56, 57, 128, 129, 160, 191, 192])
+@pytest.mark.parametrize("lens", ["uneven", "equal", "one long"])
+def test_decode_longest_first_does_not_show(batch, lens):
+    """From 56 requests of 8 kv heads to 192 the requests go by length if they hold 96 tiles each on average and one of
+    them 5/4 of the mean.  The same requests in a batch of 193 go in batch order: equal results bit for bit.  Empty and
+    equal requests among them; pages are shared between requests, which a cache of prefixes does too."""
+    from loquetier_b200 import kvcache
+    N, group, P, dtype = 8, 1, 16, torch.bfloat16
+    edge = [0, 1, 17, 4100, 1600, 1600, 3000, 2999, 64, 2500, 4100, 1023, 3300]
+    seqlens = {"uneven": (edge * 15)[:batch], "equal": [1600] * batch, "one long": [1600] * (batch - 1) + [2100]}[lens]
+    while sum(-(-n // P) for n in seqlens) * P < 96 * 16 * batch:   # raise the mean over the line
+        seqlens[seqlens.index(min(v for v in seqlens if v > 64))] = 4000
+    assert lens == "equal" or max(seqlens) * batch > 1.25 * sum(seqlens)
+    more = seqlens + [1600] * (193 - batch)
+    g = torch.Generator().manual_seed(batch)
+    pool = torch.randn((400, 1, 2, N, P, 128), generator=g).to(dtype)
+    dev = pool.to(DEV)
+    pick = [torch.randint(0, 400, (-(-n // P),), generator=g).tolist() for n in more]
+    q = torch.randn((193, N * group, 128), generator=g).to(dtype)
+
+    def run(lengths):
+        idx = [i for p in pick[:len(lengths)] for i in p]
+        ind = torch.tensor([0] + np.cumsum([-(-n // P) for n in lengths]).tolist(), dtype=torch.int32, device=DEV)
+        last = torch.tensor([A.last_page_offset_of(n, P) if n else 0 for n in lengths], dtype=torch.int32, device=DEV)
+        table = torch.tensor([dev[i].data_ptr() for i in range(400)], dtype=torch.int64, device=DEV)[idx]
+        o = torch.full((len(lengths), N * group, 128), float("nan"), dtype=dtype, device=DEV)
+        word = torch.zeros(1, dtype=torch.int32, device=DEV)
+        kvcache.batch_decode_into(o, q[:len(lengths)].to(DEV), table, ind, last, 1, 0, N, THETA, P, status_word=word)
+        assert int(word.item()) == 0
+        return o.cpu()
+
+    o = run(seqlens)
+    assert torch.equal(o, run(more)[:batch])
+    some = [0, 1, 2, 3, batch - 1]
+    host = [pool[i] for b in some for i in pick[b]]
+    ind = [0] + np.cumsum([len(pick[b]) for b in some]).tolist()
+    last = [A.last_page_offset_of(seqlens[b], P) if seqlens[b] else 0 for b in some]
+    assert_close(o[some], A.batch_decode(q[some], host, ind, last, 0, THETA), what=f"{lens} {batch}")
