@@ -250,6 +250,89 @@ struct FusedJobDesc {
   int K1, N2, accumulate;
 };
 
+// A piece can be split over the KS CTAs of a cluster; pick the KS that minimises the estimated
+// time of the launch in microseconds (constants fitted to device-side timelines on B200): per
+// CTA a set-up, a read phase that is bound either by the latency of its ring stages or by what
+// one SM can ingest, the reduce across the cluster, and a write phase bound the same way.  One
+// job: waves of CTAs x time per CTA.  Several jobs: their CTAs differ in length, so the launch
+// takes the summed CTA time over the CTA slots, and never less than its longest CTA.
+int fused_split(const FusedJobDesc* jobs, int nj, int est_pieces, int r16, bool wide, int mode) {
+  // Several jobs with at least a piece per SM between them: no split.  Such a launch is bound by
+  // bandwidth as a whole, not by the length of its longest CTA, and un-split its CTAs are few enough
+  // to become resident at once, so that an independent launch behind it can move in beside them
+  // from the start (measured on the benchmark step: dV/dX of seven projections alone takes 87 us
+  // split in two and 101 us un-split, but the step is 11 us shorter un-split, because the forward
+  // launched behind it no longer waits for a second wave of CTAs).
+  if (nj > 1 && static_cast<long long>(std::max(est_pieces, 1)) * nj >= kNumSMs) return 1;
+  const int kc = 64 * fused_chunks(r16, wide);
+  const double stage_kb = 64.0 * kc * 2 / 1024.0 * 1.28, slab_kb = 64.0 * fused_slab(r16, wide) * 2 / 1024.0;
+  const int slots = kNumSMs * fused_ctas_per_sm(r16, wide);
+  int ks = 1;
+  double best = 1e30;
+  for (int k = 1; k <= 4; ++k) {
+    bool fits = true;
+    double sum = 0.0, longest = 0.0;
+    const int ctas = std::max(est_pieces, 1) * k * nj;
+    const double load = std::max(1.0, std::min<double>(ctas, slots) / kNumSMs);  // CTAs sharing one SM
+    for (int j = 0; j < nj; ++j) {
+      const FusedJobDesc& d = jobs[j];
+      const int ksteps = (d.K1 + kc - 1) / kc, nslabs = (d.N2 + fused_slab(r16, wide) - 1) / fused_slab(r16, wide);
+      if (k > 1 && ((mode != kFusedExpandOnly && ksteps < k) || (mode != kFusedShrinkOnly && nslabs < k))) fits = false;
+      const int nk = (ksteps + k - 1) / k, ns = (nslabs + k - 1) / k;
+      const double ph1 = mode == kFusedExpandOnly ? 0.0 : std::max(2.5 + 0.9 * nk, load * nk * stage_kb / 35.0);
+      const double ph3 = mode == kFusedShrinkOnly ? 0.0 : std::max(1.0 + 1.2 * ns, load * ns * slab_kb / 33.0);
+      const double ph2 = (k > 1 && mode != kFusedExpandOnly) ? 1.0 * k : 0.6;
+      const double t = 2.0 + ph1 + ph2 + ph3;
+      sum += t * std::max(est_pieces, 1) * k;
+      longest = std::max(longest, t);
+    }
+    if (!fits) break;
+    const int waves = (ctas + slots - 1) / slots;
+    const double cost = nj == 1 ? waves * longest : std::max(longest, sum / std::min(ctas, slots));
+    if (cost < best - 1e-9) {
+      best = cost;
+      ks = k;
+    }
+  }
+  return ks;
+}
+
+// Whether a launch at rank 17..64 takes the wide form.  The narrow one is faster once an SM has two of its CTAs to work
+// on for most of the launch, and slower where it has only one, whose steps are half as long.  So narrow, by its CTAs per
+// SM (c; the segments' lengths are on the device: a segment counts as its rows / 64 and half a piece, one at least):
+//   c >= 7/4 where the jobs are of one size, c >= 9/4 where they differ (the long ones start together and, sharing SMs,
+//   end the launch), c >= 15/4 for batches of up to 10 rows a segment (panels only: what a step brings in counts);
+//   below 7/4 only if its finer steps let the pieces be split further, into at least twice the CTAs (segments of more
+//   than 8 rows; gathered pieces only where the wide form would not split at all).
+// A grouped plan of segments that short is wide: how many pieces it gathers them into is not known here, often few.
+// Measured, us, wide / narrow; forward alone:
+//   64 segments of 40 rows, rank 32     seven projections (c 3.4) 158 / 135    up and down (c 1.0) 71 / 107
+//   256 one-token segments, a prompt of 2048 rows, rank 32, seven projections   431 / 369, gathered by 32 adapters 146 / 147
+//   256 one-token segments of 8 adapters, rank 32, seven projections   89 / 163
+// and whole layer passes (rank 64, seven projections):
+//   8000 tokens of 15 segments 992 / 854, 1806 of 2 segments 149 / 235, 894 of 9 segments 75 / 112
+// Over 56 layer passes (ranks 32 and 64, 130 to 9000 tokens) the rule is at most 0.5 % slower than the wide form
+// everywhere and on average 11.5 % (rank 32) and 4.7 % (rank 64) faster; a rule by the segments' mean length alone, more
+// than 8 rows: narrow, was up to 57 % slower.
+bool fused_wide(const FusedJobDesc* jobs, int nj, int T, int nseg, int grouped, int n_table, int est_pieces, int r16,
+                int mode) {
+  if (r16 != 2 && r16 != 4) return false;
+  const int kn = fused_split(jobs, nj, est_pieces, r16, false, mode), kw = fused_split(jobs, nj, est_pieces, r16, true, mode);
+  const int short_segs = grouped ? std::min(nseg, n_table) : nseg;
+  const double pieces = std::max<double>(short_segs, T / 64.0 + short_segs / 2.0);
+  const double c = pieces * kn * nj / kNumSMs;
+  bool same = true;
+  for (int j = 1; j < nj; ++j)
+    same = same && static_cast<long long>(jobs[j].K1) + jobs[j].N2 == static_cast<long long>(jobs[0].K1) + jobs[0].N2;
+  double line = same ? 1.75 : 2.25;
+  if (T <= 10LL * nseg) {
+    if (grouped) return true;
+    line = 3.75;
+  }
+  if (c >= line) return false;
+  return !(c < 1.75 && mode != kFusedShrinkOnly && kn >= 2 * kw && T > 8LL * nseg && (!grouped || kw == 1));
+}
+
 // Runs njobs jobs that share the plan, the adapter ids, the rank and the scale.  The jobs must not
 // depend on one another (none reads what another writes).  Up to kFusedMaxJobs of them share one
 // launch; the tcgen05 variant is launched once per job.
@@ -289,58 +372,10 @@ int run_fused(const FusedJobDesc* jobs, int njobs, const int32_t* ids, const flo
   // pieces the plan is expected to hold: its capacity, except that a grouped plan turns the short
   // segments of an adapter into one gather piece, so no more than one piece per adapter comes from them
   const int est_pieces = grouped ? std::min(mp, T / piece_rows_for(T) + std::min(nseg, n_table)) : mp;
-  // Ranks 17..64: the wide form for batches of short segments - kGatherMaxLen rows a segment on average, the length
-  // up to which a grouped plan gathers them - and, above rank 32, where the launch does not give every SM a CTA (its
-  // steps are short then, and nothing shares the SM); both forms measured where they are described.
-  const bool wide = (r16 == 2 || r16 == 4) &&
-                    (T <= static_cast<long long>(kGatherMaxLen) * nseg ||
-                     (r16 == 4 && static_cast<long long>(est_pieces) * std::min(njobs, kFusedMaxJobs) < kNumSMs));
-  const int kc = 64 * fused_chunks(r16, wide);
-  const double stage_kb = 64.0 * kc * 2 / 1024.0 * 1.28, slab_kb = 64.0 * fused_slab(r16, wide) * 2 / 1024.0;
-  const int slots = kNumSMs * fused_ctas_per_sm(r16, wide);
   for (int j0 = 0; j0 < njobs; j0 += kFusedMaxJobs) {
     const int nj = std::min(kFusedMaxJobs, njobs - j0);
-    // A piece can be split over the KS CTAs of a cluster; pick the KS that minimises the estimated
-    // time of the launch in microseconds (constants fitted to device-side timelines on B200): per
-    // CTA a set-up, a read phase that is bound either by the latency of its ring stages or by what
-    // one SM can ingest, the reduce across the cluster, and a write phase bound the same way.  One
-    // job: waves of CTAs x time per CTA.  Several jobs: their CTAs differ in length, so the launch
-    // takes the summed CTA time over the CTA slots, and never less than its longest CTA.
-    int ks = 1;
-    double best = 1e30;
-    for (int k = 1; k <= 4; ++k) {
-      bool fits = true;
-      double sum = 0.0, longest = 0.0;
-      const int ctas = std::max(est_pieces, 1) * k * nj;
-      const double load = std::max(1.0, std::min<double>(ctas, slots) / kNumSMs);  // CTAs sharing one SM
-      for (int j = 0; j < nj; ++j) {
-        const FusedJobDesc& d = jobs[j0 + j];
-        const int ksteps = (d.K1 + kc - 1) / kc, nslabs = (d.N2 + fused_slab(r16, wide) - 1) / fused_slab(r16, wide);
-        if (k > 1 && ((mode != kFusedExpandOnly && ksteps < k) || (mode != kFusedShrinkOnly && nslabs < k)))
-          fits = false;
-        const int nk = (ksteps + k - 1) / k, ns = (nslabs + k - 1) / k;
-        const double ph1 = mode == kFusedExpandOnly ? 0.0 : std::max(2.5 + 0.9 * nk, load * nk * stage_kb / 35.0);
-        const double ph3 = mode == kFusedShrinkOnly ? 0.0 : std::max(1.0 + 1.2 * ns, load * ns * slab_kb / 33.0);
-        const double ph2 = (k > 1 && mode != kFusedExpandOnly) ? 1.0 * k : 0.6;
-        const double t = 2.0 + ph1 + ph2 + ph3;
-        sum += t * std::max(est_pieces, 1) * k;
-        longest = std::max(longest, t);
-      }
-      if (!fits) break;
-      const int waves = (ctas + slots - 1) / slots;
-      const double cost = nj == 1 ? waves * longest : std::max(longest, sum / std::min(ctas, slots));
-      if (cost < best - 1e-9) {
-        best = cost;
-        ks = k;
-      }
-    }
-    // Several jobs with at least a piece per SM between them: no split.  Such a launch is bound by
-    // bandwidth as a whole, not by the length of its longest CTA, and un-split its CTAs are few enough
-    // to become resident at once, so that an independent launch behind it can move in beside them
-    // from the start (measured on the benchmark step: dV/dX of seven projections alone takes 87 us
-    // split in two and 101 us un-split, but the step is 11 us shorter un-split, because the forward
-    // launched behind it no longer waits for a second wave of CTAs).
-    if (nj > 1 && static_cast<long long>(std::max(est_pieces, 1)) * nj >= kNumSMs) ks = 1;
+    const bool wide = fused_wide(jobs + j0, nj, T, nseg, grouped, n_table, est_pieces, r16, mode);
+    int ks = fused_split(jobs + j0, nj, est_pieces, r16, wide, mode);
     {
       const int forced = g_cluster_split.load(std::memory_order_relaxed);
       if (forced > 0) ks = forced;

@@ -23,7 +23,7 @@
 // numerics: fp32 accumulation, MID rounded to the storage type before the second
 // product.
 //
-// One CTA per SM; one cluster of KS CTAs owns one piece.
+// One cluster of KS CTAs owns one piece; two CTAs per SM up to rank 64, one in the wide form and above (fused_chunks).
 // Phase 1 - the HBM-bound read.  Every CTA streams its slice of the K1 columns of IN
 //   through a ring of large shared-memory stages fed by a producer warp with TMA.
 //   A stage holds 64 rows x (64*CH) columns, fetched as [16 rows x 64 columns] tiled
@@ -66,14 +66,10 @@ constexpr int kFusedCThreads = kFusedConsumers * 32;
 // Ranks up to 64 are sized so that two CTAs fit on one SM: an independent successor launch can then
 // move in and read while this launch is still writing, and one CTA's set-up and turn from reading to
 // writing pass under the other's copies.  At rank 17..64 there is a second form, `wide`: one CTA per SM with twice
-// the width of a step.  Pieces of a few rows only stream panels, W1 as one copy per rank and step, and there the
-// longer copies count for more; so they do, above rank 32, in launches that have no second CTA for an SM.  Measured,
-// hidden sizes 4096 and 11008, us, wide against narrow:
-//   1024 one-token segments of 256 adapters, two projections     rank 32  191 / 204
-//   zipf lengths, seven projections, a quarter trained:
-//     8192 tokens     rank 32  485 / 408    rank 40  845 / 682    rank 64  1031 / 884
-//     1000 tokens     rank 32  102 / 92     rank 40  157 / 142    rank 64  184 / 171
-//     128 tokens      rank 32  90 / 72      rank 40  72 / 87      rank 64  77 / 102
+// the width of a step, for launches that leave an SM one CTA at a time and for gathered pieces of a few rows, which only
+// stream panels (W1 as one copy per rank and step: the longer copies count for more).  The rule between them and both
+// sides' figures stand at fused_wide.  The narrow form has 96 registers a thread and spills a little at rank 17..32
+// (20-56 bytes of stores, 40-104 of loads by instantiation; at rank 33..64 at most 12).
 constexpr int fused_chunks(int r16, bool wide) { return r16 >= 8 ? 2 : (r16 == 4 ? (wide ? 4 : 2) : (wide ? 8 : 4)); }
 constexpr int fused_stages(int) { return 2; }
 constexpr int fused_slab(int r16, bool wide) { return r16 >= 8 ? 128 : (r16 == 4 ? 256 : (wide ? 1024 : 512)); }
@@ -469,8 +465,9 @@ __global__ void __launch_bounds__(kFusedThreads, fused_ctas_per_sm(R16, WIDE)) f
                    "r"(packed));
     }
   }
-  // done reading the peers' partial sums; the matching wait sits at the very end, so that no CTA
-  // leaves (and frees its shared memory) while a peer may still be reading it
+  // done reading the peers' partial sums; the matching wait keeps a CTA from leaving (and freeing its shared memory)
+  // while a peer may still be reading it.  It sits at the very end, except in the narrow form of rank 17..64, whose
+  // write phase reuses that memory: there it comes right below
   if (reduce_cluster) cluster_arrive();
   __syncthreads();  // MID is complete; the ring is free for phase 3
   if constexpr (SM::kRedInRing) {
