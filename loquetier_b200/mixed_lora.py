@@ -18,7 +18,7 @@ from torch import nn
 from torch.autograd.function import Function
 
 from . import ops
-from .kernel_utils import BatchLenInfo, _ptr_table, _ptr_tables, add_lora
+from .kernel_utils import BatchLenInfo, _ptr_tables, add_lora
 from .segments import wants_grouped_plan
 
 
@@ -160,13 +160,15 @@ class MixedLoraLinear(nn.Module):
 
     # -- pointer tables (mixed_lora.py:106-166) ---------------------------------
     def _refresh_tables(self):
-        self.wa_ptrs = _ptr_table([a.wa for a in self.adapters], self.device)
-        self.wb_ptrs = _ptr_table([a.wb for a in self.adapters], self.device)
+        # These tables live as long as the module and are read on whatever stream runs it, which need not be the one
+        # they are made on: copies that the host waits for, so that they are complete on return.
+        self.wa_ptrs = torch.tensor([a.wa.data_ptr() for a in self.adapters], dtype=torch.int64, device=self.device)
+        self.wb_ptrs = torch.tensor([a.wb.data_ptr() for a in self.adapters], dtype=torch.int64, device=self.device)
         if not self.is_scaled:
-            vals = [a.scaling for a in self.adapters]
-            self.scaling = torch.tensor(vals, dtype=self.dtype, device=self.device)
+            scaling = torch.tensor([a.scaling for a in self.adapters], dtype=self.dtype)
+            self.scaling = scaling.to(self.device)
             # the kernels take the scale in fp32; it carries the module dtype's rounding
-            self.scaling_f32 = self.scaling.to(torch.float32)
+            self.scaling_f32 = scaling.to(torch.float32).to(self.device)
 
     def update_adapters(self, adapters: List[NamedLoraLayer], rank: int):
         self.adapters = adapters
