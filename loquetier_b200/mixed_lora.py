@@ -52,18 +52,23 @@ class MixedLoraContext:
 
     def device_state(self, device: torch.device, T: int) -> dict:
         """Segment index pointer, adapter index per segment, train partitions and
-        their plans on ``device``; built on first use after ``update``."""
+        their plans on ``device``; built on first use after ``update``, never under stream capture: a capture would
+        record the launches that fill it, run none of them, and leave it to later calls outside the graph."""
         key = (device, int(T))
         st = self._dev.get(key)
         if st is None:
+            if device.type == "cuda":
+                with torch.cuda.device(device):
+                    if torch.cuda.is_current_stream_capturing():
+                        raise RuntimeError("the first forward after MixedLoraContext.update() builds the batch's device "
+                                           "state and cannot be captured in a CUDA graph; run one before the capture")
             seg = self._segment.to(device=device, dtype=torch.int32).contiguous()
             ids = list(self._lora_ids)
             seg_ids = ops.device_ints(ids, torch.int32, device)
             # grouped plan when it helps: decode tokens of one adapter then share its panels wherever they
             # sit in the batch.  Only an adapter with several segments can ask for it; then the segments' lengths
             # are needed.  The reference keeps `segment` on the device (model_generation.py:279-283): they come
-            # back in ONE copy, outside any stream capture (the state is built on the first forward after
-            # `update`), never element by element.
+            # back in ONE copy, never element by element.
             grouped = False
             if len(set(ids)) < len(ids):
                 bounds = self._segment.tolist()

@@ -42,3 +42,36 @@ def test_a_modules_tables_are_complete_on_return(is_scaled):
         if not is_scaled:
             assert lin.scaling_f32.tolist() == [float(torch.tensor(a.scaling).to(torch.bfloat16)) for a in lin.adapters]
     side.synchronize()
+
+
+def _batch(ctx, lens, ids, trains, train_idx):
+    from loquetier_b200.kernel_utils import BatchLenInfo
+    seg = torch.tensor([0] + torch.tensor(lens).cumsum(0).tolist(), dtype=torch.int32, device=DEV)
+    blen = BatchLenInfo([(1, n) for n in lens[:trains]], [], sum(lens[trains:]), [], DEV)
+    ctx.update(blen, ids, torch.tensor(lens, dtype=torch.int32, device=DEV), seg, train_idx)
+
+
+@pytest.mark.parametrize("trains", [0, 2])
+def test_the_first_forward_of_a_batch_is_refused_under_capture(trains):
+    """It builds the batch's plans and index arrays, which later forwards use outside the graph as well; under capture
+    nothing of it would have run.  The batch is as before afterwards, and a captured forward after an eager one works."""
+    ctx, _, _, make = _module(4)
+    lin = make()
+    lin.set_trainable([0, 1])
+    lens, ids = [20, 30, 1, 1], [0, 1, 2, 3]
+    _batch(ctx, lens, ids, trains, [0, 1][:trains])
+    x = torch.randn((sum(lens), 64), device=DEV).to(torch.bfloat16)
+    graph = torch.cuda.CUDAGraph()
+    with torch.no_grad():
+        lin.base_layer(x)   # (the base product's library is set up)
+        with pytest.raises(RuntimeError, match="captur"):
+            with torch.cuda.graph(graph):
+                lin(x)
+        assert ctx._dev == {}
+        want = lin(x)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            got = lin(x)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(got, want)
