@@ -119,6 +119,8 @@ class add_lora(Function):
         if tl == 0:
             return (None, grad_x, None, None, None, None, None, None,
                     *[torch.zeros_like(w) for w in weight_list])
+        # the tables below carry the addresses of this call's gradients and weights, which a graph would replay
+        ops.refuse_capture(go, "the backward of add_lora")
         part = ops.device_ints([int(t) for t in tp[:npart + 1]], torch.int32, dev)
         plan = ops.Plan(part, tl)
         was, wbs = weight_list[0:2 * npart:2], weight_list[1:2 * npart:2]

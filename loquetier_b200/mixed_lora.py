@@ -137,6 +137,8 @@ class _lora_linear_fn(Function):
         grad_x = torch.zeros((go.size(0), x.size(1)), dtype=go.dtype, device=go.device)
         grads: List[Optional[torch.Tensor]] = [None] * ctx.ntrain
         if tl > 0 and ctx.ntrain > 0:
+            # the tables below carry the addresses of this call's gradients, which a graph would replay
+            ops.refuse_capture(go, "the backward of a MixedLoraLinear with trained adapters")
             npart = ctx.ntrain // 2
             dA = [torch.empty_like(mod.adapters[i].wa) for i in mod.root_context.train_idx[:npart]]
             dB = [torch.empty_like(mod.adapters[i].wb) for i in mod.root_context.train_idx[:npart]]

@@ -46,6 +46,15 @@ def on_device(t: torch.Tensor):
     return _SAME_DEVICE if i >= 0 and i == torch.cuda.current_device() else torch.cuda.device(t.device)
 
 
+def refuse_capture(t: torch.Tensor, what: str):
+    """Raises if the current stream of the tensor's device is being captured: for calls whose arrays on the device
+    describe this very call."""
+    if t.is_cuda:
+        with on_device(t):
+            if torch.cuda.is_current_stream_capturing():
+                raise RuntimeError(f"{what} cannot be captured in a CUDA graph")
+
+
 _UPLOAD_LIMIT = 1 << 14   # bytes; above, one pageable copy costs less than the launches
 
 

@@ -75,3 +75,38 @@ def test_the_first_forward_of_a_batch_is_refused_under_capture(trains):
     graph.replay()
     torch.cuda.synchronize()
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("kind", ["linear", "add_lora"])
+def test_a_backward_is_refused_under_capture(kind):
+    """It writes the addresses of this call's gradients and weights to the device; a graph would keep them.  The same
+    backward runs afterwards outside the capture."""
+    from loquetier_b200.kernel_utils import add_lora
+    ctx, _, ads, make = _module(4)
+    lens, ids = [20, 30, 1, 1], [0, 1, 2, 3]
+    x = torch.randn((sum(lens), 64), device=DEV).to(torch.bfloat16).requires_grad_(True)
+    go = torch.randn((sum(lens), 96), device=DEV).to(torch.bfloat16)
+    lin = make()
+    lin.set_trainable([0, 1])
+    params = [lin.get_parameter(f"lora-{i}-{k}") for i in (0, 1) for k in "AB"]
+    _batch(ctx, lens, ids, 2, [0, 1])
+    tab = lambda k: torch.tensor([getattr(ads[i], k).data_ptr() for i in ids], dtype=torch.int64, device=DEV)
+    seg = torch.tensor([0, 20, 50, 51, 52], dtype=torch.int32, device=DEV)
+    wa, wb = tab("wa"), tab("wb")
+
+    def forward():
+        if kind == "linear":
+            return lin(x)
+        return add_lora.apply((sum(lens), 96), x, wa, wb, seg, 8, 50, [0, 20, 50], *params)
+
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        want = torch.autograd.grad(forward(), [x] + params, go)
+        y = forward()
+        with pytest.raises(RuntimeError, match="captur"):
+            with torch.cuda.graph(torch.cuda.CUDAGraph(), stream=side):
+                torch.autograd.grad(y, [x] + params, go, retain_graph=True)
+        got = torch.autograd.grad(y, [x] + params, go)
+    side.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(want, got))
