@@ -17,7 +17,7 @@ import torch
 
 from . import cabi
 from .cabi import check, lib
-from .ops import _stream, on_device
+from .ops import _stream, on_device, workspace_uncleared
 
 _DT = {torch.float16: cabi.SMLM_F16, torch.bfloat16: cabi.SMLM_BF16}
 
@@ -155,6 +155,7 @@ class BatchedKvCache:
 
 _WORKSPACES = {}
 _WS_HEAD = {}   # device -> bytes of tickets at the head of the workspace for the batch it last served
+_WS_RECORDED = set()   # devices whose workspace was made under capture (ops.workspace_uncleared)
 
 
 def _dtype_code(t):
@@ -176,7 +177,8 @@ def decode_workspace(device, batch: int, num_qo_heads: int, num_kv_heads: int) -
     if ws is None or ws.numel() < need:
         ws = torch.zeros(max(need, 1 << 16), dtype=torch.uint8, device=device)
         _WORKSPACES[device] = ws
-    elif _WS_HEAD.get(device) != head and head > 0:
+        workspace_uncleared(_WS_RECORDED, device, ws, fresh=True)
+    elif workspace_uncleared(_WS_RECORDED, device, ws, fresh=False) or _WS_HEAD.get(device) != head:
         with on_device(ws):
             ws[:head].zero_()
     _WS_HEAD[device] = head

@@ -202,6 +202,23 @@ _WORKSPACES = {}
 
 
 _WS_SHAPE = {}   # (device, slot) -> (shape, bytes of tickets) the cached workspace was last handed out for
+_WS_RECORDED = set()   # keys whose workspace was made under capture: its zeros are recorded there, not yet on the device
+
+
+def workspace_uncleared(recorded: set, key, ws: torch.Tensor, fresh: bool) -> bool:
+    """Whether the head of a cached workspace has to be cleared because the zeros it was made with may never have been
+    written: it was made under stream capture, and only a replay writes them.  A call outside a capture clears it for
+    good; a captured one for its own graph."""
+    if not ws.is_cuda or (not fresh and key not in recorded):
+        return False
+    with on_device(ws):
+        capturing = torch.cuda.is_current_stream_capturing()
+    if fresh:
+        (recorded.add if capturing else recorded.discard)(key)
+        return False
+    if not capturing:
+        recorded.discard(key)
+    return True
 
 
 def _cached_workspace(device, slot, need: int, shape, ticket_bytes: int) -> torch.Tensor:
@@ -214,9 +231,11 @@ def _cached_workspace(device, slot, need: int, shape, ticket_bytes: int) -> torc
     if ws is None or ws.numel() < need:
         ws = torch.zeros(max(need, 1 << 20), dtype=torch.uint8, device=device)
         _WORKSPACES[key] = ws
+        workspace_uncleared(_WS_RECORDED, key, ws, fresh=True)
     else:
         prev_shape, prev_bytes = _WS_SHAPE[key]
-        if prev_shape != shape and max(prev_bytes, ticket_bytes) > cabi.SMLM_TICKET_HEAD:
+        moved = prev_shape != shape and max(prev_bytes, ticket_bytes) > cabi.SMLM_TICKET_HEAD
+        if workspace_uncleared(_WS_RECORDED, key, ws, fresh=False) or moved:
             with on_device(ws):
                 ws[:ticket_bytes].zero_()
     _WS_SHAPE[key] = (shape, ticket_bytes)

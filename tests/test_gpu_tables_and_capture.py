@@ -110,3 +110,54 @@ def test_a_backward_is_refused_under_capture(kind):
         got = torch.autograd.grad(y, [x] + params, go)
     side.synchronize()
     assert all(torch.equal(a, b) for a, b in zip(want, got))
+
+
+def test_a_workspace_made_under_capture_is_cleared_before_its_first_eager_use():
+    """The zeros of a workspace that a capture allocates are recorded there; until a replay its memory holds anything."""
+    from loquetier_b200 import kvcache, ops
+    N, group, P = 8, 4, 16
+    g = torch.Generator(device=DEV).manual_seed(3)
+    pool = torch.randn((400, 1, 2, N, P, 128), generator=g, device=DEV).to(torch.bfloat16)
+
+    def decode(batch, pages):
+        ptrs = torch.tensor([pool[i].data_ptr() for i in range(batch * pages)], dtype=torch.int64, device=DEV)
+        ind = torch.arange(0, (batch + 1) * pages, pages, dtype=torch.int32, device=DEV)
+        last = torch.full((batch,), P, dtype=torch.int32, device=DEV)
+        q = torch.randn((batch, N * group, 128), generator=g, device=DEV).to(torch.bfloat16)
+        o = torch.full_like(q, float("nan"))
+        return o, lambda: kvcache.batch_decode_into(o, q, ptrs, ind, last, 1, 0, N, 1e4, P)
+
+    def wgrad(npart, rows, hi, ho, rank):
+        n = npart * rows
+        rnd = lambda *s: torch.randn(s, generator=g, device=DEV).to(torch.bfloat16)
+        x, go, v, dv = rnd(n, hi), rnd(n, ho), rnd(n, rank), rnd(n, rank)
+        out = torch.full((npart, rank * (hi + ho)), float("nan"), dtype=torch.bfloat16, device=DEV)
+        part = torch.arange(0, n + 1, rows, dtype=torch.int32, device=DEV)
+        tab = lambda off: torch.tensor([o.data_ptr() + 2 * off for o in out], dtype=torch.int64, device=DEV)
+        tA, tB, plan = tab(0), tab(rank * hi), ops.Plan(part, n)
+        return out, lambda: ops.wgrad_pair(tA, tB, dv, x, v, go, part, plan, rank)
+
+    # the first of each pair needs the larger workspace
+    for caches, a, b in (((kvcache._WORKSPACES,), decode(4, 80), decode(3, 60)),
+                         ((ops._WORKSPACES,), wgrad(3, 700, 1024, 512, 16), wgrad(2, 600, 512, 256, 8))):
+        want = []
+        for out, run in (a, b):
+            run()
+            torch.cuda.synchronize()
+            want.append(out.clone())
+            out.fill_(float("nan"))
+        for cache in caches:
+            cache.clear()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            a[1]()
+        for ws in caches[0].values():
+            ws.fill_(1)                      # what memory holds that nothing has cleared
+        for out, run in (b, a):
+            run()
+        torch.cuda.synchronize()
+        assert torch.equal(a[0], want[0]) and torch.equal(b[0], want[1])
+        a[0].fill_(float("nan"))
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(a[0], want[0])
