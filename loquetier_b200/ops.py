@@ -64,7 +64,10 @@ def device_ints(values, dtype: torch.dtype, device) -> torch.Tensor:
     device = torch.device(device)
     if device.type != "cuda" or not 0 < len(values) <= _UPLOAD_LIMIT // 8:
         return torch.tensor(values, dtype=dtype, device=device)
-    host = array.array("q" if dtype == torch.int64 else "i", values)
+    try:
+        host = array.array("q" if dtype == torch.int64 else "i", values)
+    except (TypeError, OverflowError):   # what torch.tensor converts, or refuses in its own words
+        return torch.tensor(values, dtype=dtype, device=device)
     t = torch.empty(len(host), dtype=dtype, device=device)
     with on_device(t):
         check(lib.smlm_b200_upload(t.data_ptr(), host.buffer_info()[0], len(host) * host.itemsize, _stream(t)),

@@ -161,3 +161,15 @@ def test_a_workspace_made_under_capture_is_cleared_before_its_first_eager_use():
         graph.replay()
         torch.cuda.synchronize()
         assert torch.equal(a[0], want[0])
+
+
+def test_device_ints_takes_what_torch_tensor_takes():
+    from loquetier_b200 import ops
+    for vals in ([True, False], [1.0, 2.0, -3.0], [torch.tensor(4), torch.tensor(5)], torch.tensor([6, 7]), (8, 9)):
+        for dtype in (torch.int32, torch.int64):
+            assert ops.device_ints(vals, dtype, DEV).tolist() == torch.tensor(list(vals), dtype=dtype).tolist()
+    for bad, dtype in (([1 << 31], torch.int32), ([1 << 63], torch.int64), (["a"], torch.int32), ([None], torch.int32)):
+        with pytest.raises((RuntimeError, TypeError, ValueError, OverflowError)) as want:
+            torch.tensor(bad, dtype=dtype, device=DEV)
+        with pytest.raises(want.type):
+            ops.device_ints(bad, dtype, DEV)
