@@ -209,10 +209,11 @@ int smlm_b200_wgrad(void* const* g_table, const void* p, const void* q, const in
  * library's device image instead and calls no allocating routine at all.
  *
  * Same arguments and results as smlm_b200_wgrad, minus the workspace.  Limits and rules:
- *  - the array is SMLM_STATIC_WGRAD_BYTES (16 MiB) and every GPU that loads the library
- *    holds it until the process exits; a problem whose workspace
- *    (smlm_b200_wgrad_workspace_bytes(T, npart, rank, h, 0)) is larger is refused with
- *    SMLM_ERR_STATIC_LIMIT before anything is launched;
+ *  - the array holds SMLM_STATIC_WGRAD_BYTES (16 MiB) and the smallest ticket head (SMLM_TICKET_HEAD) on top, and
+ *    every GPU that loads the library holds it until the process exits; a problem whose tickets and parked sums
+ *    together take more than SMLM_STATIC_WGRAD_BYTES is refused with SMLM_ERR_STATIC_LIMIT before anything is
+ *    launched.  None is whose smlm_b200_wgrad_workspace_bytes(T, npart, rank, h, 0), which counts a whole head, is
+ *    no larger than that;
  *  - the first call on each device looks up the array's device address (with that
  *    device current).  Make that first call outside any stream capture;
  *  - all calls on a device share the one array, which keeps the previous call's

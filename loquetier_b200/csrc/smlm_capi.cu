@@ -1037,7 +1037,7 @@ int smlm_b200_wgrad_static(void* const* g_table, const void* p, const void* q, c
   if (rc != SMLM_OK) return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   // the array keeps whatever the previous call left; only the tickets have to start at zero
-  if (cudaMemsetAsync(scratch, 0, sh.ticket_bytes, st) != cudaSuccess) {
+  if (cudaMemsetAsync(scratch, 0, sh.tickets_used, st) != cudaSuccess) {
     cudaGetLastError();
     return SMLM_ERR_CUDA;
   }
