@@ -17,7 +17,7 @@ import torch
 
 from . import cabi
 from .cabi import check, lib
-from .ops import _stream, on_device, workspace_uncleared
+from .ops import _stream, clear_recorded_workspace, note_fresh_workspace, on_device
 
 _DT = {torch.float16: cabi.SMLM_F16, torch.bfloat16: cabi.SMLM_BF16}
 
@@ -155,7 +155,7 @@ class BatchedKvCache:
 
 _WORKSPACES = {}
 _WS_HEAD = {}   # device -> bytes of tickets at the head of the workspace for the batch it last served
-_WS_RECORDED = set()   # devices whose workspace was made under capture (ops.workspace_uncleared)
+_WS_RECORDED = set()   # devices whose workspace was made under capture (ops.clear_recorded_workspace)
 
 
 def _dtype_code(t):
@@ -177,8 +177,10 @@ def decode_workspace(device, batch: int, num_qo_heads: int, num_kv_heads: int) -
     if ws is None or ws.numel() < need:
         ws = torch.zeros(max(need, 1 << 16), dtype=torch.uint8, device=device)
         _WORKSPACES[device] = ws
-        workspace_uncleared(_WS_RECORDED, device, ws, fresh=True)
-    elif workspace_uncleared(_WS_RECORDED, device, ws, fresh=False) or _WS_HEAD.get(device) != head:
+        note_fresh_workspace(_WS_RECORDED, device, ws)
+    elif device in _WS_RECORDED:
+        clear_recorded_workspace(_WS_RECORDED, device, ws, head)
+    elif _WS_HEAD.get(device) != head:
         with on_device(ws):
             ws[:head].zero_()
     _WS_HEAD[device] = head

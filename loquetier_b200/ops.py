@@ -208,20 +208,22 @@ _WS_SHAPE = {}   # (device, slot) -> (shape, bytes of tickets) the cached worksp
 _WS_RECORDED = set()   # keys whose workspace was made under capture: its zeros are recorded there, not yet on the device
 
 
-def workspace_uncleared(recorded: set, key, ws: torch.Tensor, fresh: bool) -> bool:
-    """Whether the head of a cached workspace has to be cleared because the zeros it was made with may never have been
-    written: it was made under stream capture, and only a replay writes them.  A call outside a capture clears it for
-    good; a captured one for its own graph."""
-    if not ws.is_cuda or (not fresh and key not in recorded):
-        return False
+def note_fresh_workspace(recorded: set, key, ws: torch.Tensor):
+    """Keeps in ``recorded`` whether the zeros of a workspace just made are only recorded so far."""
+    recorded.discard(key)
+    if ws.is_cuda:
+        with on_device(ws):
+            if torch.cuda.is_current_stream_capturing():
+                recorded.add(key)
+
+
+def clear_recorded_workspace(recorded: set, key, ws: torch.Tensor, head: int):
+    """Clears the head of a workspace that was made under capture, where only a replay writes its zeros: a call outside
+    a capture for good, a captured one for its own graph."""
     with on_device(ws):
-        capturing = torch.cuda.is_current_stream_capturing()
-    if fresh:
-        (recorded.add if capturing else recorded.discard)(key)
-        return False
-    if not capturing:
-        recorded.discard(key)
-    return True
+        ws[:head].zero_()
+        if not torch.cuda.is_current_stream_capturing():
+            recorded.discard(key)
 
 
 def _cached_workspace(device, slot, need: int, shape, ticket_bytes: int) -> torch.Tensor:
@@ -234,11 +236,12 @@ def _cached_workspace(device, slot, need: int, shape, ticket_bytes: int) -> torc
     if ws is None or ws.numel() < need:
         ws = torch.zeros(max(need, 1 << 20), dtype=torch.uint8, device=device)
         _WORKSPACES[key] = ws
-        workspace_uncleared(_WS_RECORDED, key, ws, fresh=True)
+        note_fresh_workspace(_WS_RECORDED, key, ws)
+    elif key in _WS_RECORDED:
+        clear_recorded_workspace(_WS_RECORDED, key, ws, ticket_bytes)
     else:
         prev_shape, prev_bytes = _WS_SHAPE[key]
-        moved = prev_shape != shape and max(prev_bytes, ticket_bytes) > cabi.SMLM_TICKET_HEAD
-        if workspace_uncleared(_WS_RECORDED, key, ws, fresh=False) or moved:
+        if prev_shape != shape and max(prev_bytes, ticket_bytes) > cabi.SMLM_TICKET_HEAD:
             with on_device(ws):
                 ws[:ticket_bytes].zero_()
     _WS_SHAPE[key] = (shape, ticket_bytes)
