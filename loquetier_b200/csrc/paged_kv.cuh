@@ -168,12 +168,12 @@ __device__ __forceinline__ void turn_f32x2(uint64_t& c, uint64_t& s, uint64_t c1
 //
 // What bounds it: with the keys' rows rotated in place in shared memory (two loads and two stores per key and
 // lane) and the heads as the rows of a half-empty tile, a tile of 16 keys took a warp about 960 instructions and
-// the 12 warps of an SM could not issue them as fast as the keys arrive; this form needs a little over half.  The
-// maxima are exchanged (six shuffles) and the sums rescaled only in tiles that raise one, which a vote finds out.  They
-// are raised by any excess: the weights are rounded to 16 bits, and the key that sets the maximum has the weight one
-// exactly.  Raising them late, at an excess of 2^8, made the results' error against 64 bits 3-5 % larger.
-// Measured, append + decode of 128 requests with contexts 512..4096, 32 / 8 heads (1236 MB): 287 us before, 215 us
-// now (5.75 TB/s), with the longest requests first.
+// the 12 warps of an SM could not issue them as fast as the keys arrive; this form takes about 660.  The maxima are
+// exchanged (six shuffles) and the sums rescaled only in tiles that raise one, which a vote finds out.  They are raised by
+// any excess: the weights are rounded to 16 bits, and the key that sets the maximum has the weight one exactly.  Raising
+// them late, at an excess of 2^8, made the results' error against 64 bits 2.4 % larger (geometric mean, up to 7.5 %).
+// Measured, append + decode of 128 requests with contexts 512..4096 drawn evenly, 32 / 8 heads (1236 MB), longest first:
+// 287 us before, 217 us now (5.7 TB/s) as one call among others on new inputs; 199-210 us replayed from a graph.
 template <typename T, int G>
 __global__ void __launch_bounds__(kPdWarps * 32, 3) paged_decode_kernel(const PdArgs a) {
   extern __shared__ __align__(128) unsigned char pd_smem[];
@@ -246,7 +246,7 @@ __global__ void __launch_bounds__(kPdWarps * 32, 3) paged_decode_kernel(const Pd
   const int ntl = max(0, min(ntiles, tile0 + per) - tile0);   // tiles of this CTA
   const int ntw = ntl > warp ? (ntl - warp + kPdWarps - 1) / kPdWarps : 0;   // tiles of this warp
 
-  // ---- the rotated, pre-scaled queries as the A operand: [8 rows][128] in shared memory ----
+  // ---- the rotated, pre-scaled queries, the B operand: [8 rows][128] in shared memory ----
   // Angles are kept in half-turns (angle / pi): sincospif reduces its argument exactly, whereas the
   // library is built with fast math, under which sincosf loses accuracy at the angles long sequences reach.
   const uint32_t sbase = smem_u32(pd_smem);

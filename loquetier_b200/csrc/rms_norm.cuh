@@ -266,7 +266,8 @@ __global__ void __launch_bounds__(kRmsThreads) rms_norm_dw_kernel(void* __restri
   float s = 0.f;
   if (col < cols) {
     // Bound by latency (a few hundred partials, one column per thread): sixteen are requested together and added
-    // in order (32768 x 4096, forward and backward: 236.0 -> 234.9 us).
+    // in order.  Within the noise of the pass (32768 x 4096, forward and backward: 236.0 and 234.9 us, 240 and 238 on another
+    // card); the launch itself is a few us.
     constexpr int U = 16, STEP = kRmsThreads / 32;
     const float* src = partial + static_cast<size_t>(warp) * cols + col;
     const size_t stride = static_cast<size_t>(STEP) * cols;
