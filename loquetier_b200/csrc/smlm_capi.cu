@@ -311,7 +311,7 @@ int fused_split(const FusedJobDesc* jobs, int nj, int est_pieces, int r16, bool 
 //   256 one-token segments of 8 adapters, rank 32, seven projections   89 / 163
 // and whole layer passes (rank 64, seven projections):
 //   8000 tokens of 15 segments 992 / 854, 1806 of 2 segments 149 / 235, 894 of 9 segments 75 / 112
-// Over 56 layer passes (ranks 32 and 64, 130 to 9000 tokens) the rule is at most 0.5 % slower than the wide form
+// Over 56 layer passes (ranks 32 and 64, 130 to 9000 tokens) the rule is at most 1 % slower than the wide form
 // everywhere and on average 11.5 % (rank 32) and 4.7 % (rank 64) faster; a rule by the segments' mean length alone, more
 // than 8 rows: narrow, was up to 57 % slower.
 bool fused_wide(const FusedJobDesc* jobs, int nj, int T, int nseg, int grouped, int n_table, int est_pieces, int r16,
